@@ -1,0 +1,469 @@
+// Gauss-Seidel sweep and residual of the levels whose rows are stored per node
+// (OP_DENSE: Galerkin levels of variable coefficients, per-node stencils).
+//
+// A row is 26 neighbour blocks of 9 coefficients, 1 or 2 KB per node.  Large
+// levels are bound by those bytes (FP32) or by the FP64 pipe, small ones, with
+// few nodes per colour, by latency.  A thread per node does badly at all three:
+// so the blocks of a row are spread over the warps of a CTA, lanes along the
+// nodes (coalesced), and the parts are summed through shared memory in the
+// order of dense_row (ops.cuh), which the colour launches use: the results are
+// equal bit for bit.
+//
+//  * FP32: 32 nodes at a time, 13 warps with two blocks each; a 14th warp sums
+//    the 26 products of a node and applies the inverse centre block.
+//  * FP64: an SM scheduler issues an FP64 instruction every 64 cycles, whether
+//    its warp has one active lane or 32 (measured), so the four schedulers
+//    have to be loaded alike and the lanes filled: a team of four warps takes
+//    10 nodes, a lane per node and row, a warp per part of dense_row (7, 6, 7
+//    and 6 blocks), and the warps take turns at the sums.
+//
+// The sweep is two launches, the even planes and then the odd ones (colours
+// 0-3 and 4-7; region::gauss_seidel, mg_3d_template/region.cc:1557-1762, in
+// the 8-colour order).  A cluster of up to 8 CTAs runs the four colours of one
+// plane, with a cluster barrier between two colours.  What does not depend on
+// the colour before is loaded ahead of the barrier: the coefficients, and x of
+// the planes above and below.
+//
+// One sweep on GB300, before (one block a plane on planes of up to 64x64,
+// else eight colour launches, a thread a node) and now:
+//   64x64x65  FP32  310 -> 97 us     16x16x17  FP32   54 -> 20 us
+//   49x41x33  FP64  328 -> 180 us    32x48x26  FP64  245 -> 84 us
+//   7x6x5     FP64  118 -> 38 us
+// and the residual of 49x41x33 in FP64 72 -> 65 us, of 16x16x17 in FP32 23 -> 3 us.
+#include <algorithm>
+
+#include "launch.h"
+#include "ops.cuh"
+
+namespace stzmg {
+
+namespace {
+
+constexpr int kOut = INT32_MIN / 4;   // outside a non-periodic grid
+
+// Slot offset of the neighbour d of sub-grid coordinate I (parity a) along one
+// dimension: one entry of dim_offsets.
+__device__ __forceinline__ int dim_off(int I, int a, int n, int N2, int prd, int pstride, int istride, int d) {
+    const int own = a * pstride + I * istride;
+    if (d == 0) return own;
+    if (n == 1) return prd ? own : kOut;
+    if (d < 0) return a ? I * istride : I > 0 ? pstride + (I - 1) * istride : prd ? pstride + (N2 - 1) * istride : kOut;
+    return 2 * I + a + 1 < n ? (a ? (I + 1) * istride : pstride + I * istride) : prd ? 0 : kOut;
+}
+
+// Slot of the neighbour through block b of node (I, J, K) of colour q; negative outside the grid.
+__device__ __forceinline__ int block_slot(const Geom &g, int I, int J, int K, int q, int b) {
+    return dim_off(I, q & 1, g.m, g.M2, g.xp, g.S, 1, b % 3 - 1) +
+           dim_off(J, (q >> 1) & 1, g.n, g.N2, g.yp, 2 * g.S, g.M2, (b / 3) % 3 - 1) +
+           dim_off(K, q >> 2, g.o, g.O2, g.zp, 4 * g.S, g.M2 * g.N2, b / 9 - 1);
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// ---------------------------------------------------------------- FP32
+constexpr int kDotWarps = 13;                        // two blocks each: b and 26 - b
+constexpr int kThreads32 = 32 * (kDotWarps + 1);     // the last warp sums
+
+using DotTable = float[26][3][32];
+
+// What a dot warp holds of its two blocks for one node per lane.
+struct BlockPair {
+    float a[2][9], v[2][3];
+    int s[2];
+
+    // coefficients of blocks w and 26 - w at slot p, and the neighbours' slots
+    __device__ __forceinline__ void load(const DenseOp<float> &op, const Geom &g, bool valid, int w, int I, int J,
+                                         int K, int q, int p) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int b = u ? 26 - w : w;
+            s[u] = valid ? block_slot(g, I, J, K, q, b) : -1;
+            const float *cb = op.coef + (size_t)(9 * b) * g.npad + p;
+#pragma unroll
+            for (int e = 0; e < 9; e++) a[u][e] = s[u] >= 0 ? __ldg(cb + (size_t)e * g.npad) : 0.0f;
+        }
+    }
+    template <bool COH>
+    __device__ __forceinline__ void load_x(const float *x, int npad) {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            if (s[u] >= 0) load3<float, COH>(x, npad, s[u], v[u]);
+            else v[u][0] = v[u][1] = v[u][2] = 0.0f;
+        }
+    }
+    // the products, into the CTA's table (0 for a neighbour outside the grid)
+    __device__ __forceinline__ void dots(int w, int lane, DotTable &out) const {
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            float(*o)[32] = out[u ? 25 - w : w];
+#pragma unroll
+            for (int r = 0; r < 3; r++)
+                o[r][lane] = dot3(a[u][3 * r], v[u][0], a[u][3 * r + 1], v[u][1], a[u][3 * r + 2], v[u][2]);
+        }
+    }
+};
+
+// Colours 4c .. 4c+3 of every plane of parity c, `cl` CTAs (one cluster) per
+// plane; x is updated in place.
+__global__ void __launch_bounds__(kThreads32)
+    gs_dense32_kernel(Geom g, int c, int cl, DenseOp<float> op, const float *__restrict__ r, float *x) {
+    __shared__ DotTable dots[2];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int rank = blockIdx.x % cl, K = blockIdx.x / cl;
+    const int plane = g.M2 * g.N2, per = ((plane + 31) / 32 + cl - 1) / cl;
+    const bool sums = wid == kDotWarps;
+    const bool inplane = wid >= 9;   // blocks 9 .. 12 and 14 .. 17; the other warps read the planes above and below
+    const size_t np = (size_t)g.npad;
+    BlockPair row;
+    float acc[3], inv[9];
+    int p = -1;   // the summing warp's node
+    // item w: the (w % per)-th 32 nodes of this CTA in colour w / per of the plane
+    auto load = [&](int w) {
+        const int q = 4 * c + w / per, t = 32 * (rank + cl * (w % per)) + lane;
+        const int J = t / g.M2, I = t - J * g.M2;
+        const bool valid = t < plane && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n;
+        const int s = q * g.S + K * plane + t;
+        if (!sums) {
+            row.load(op, g, valid, wid, I, J, K, q, s);
+            // a colour's own plane is final once the colour before it is done
+            if (!inplane || w % per != 0) row.load_x<true>(x, g.npad);
+        } else {
+            p = valid ? s : -1;
+            if (valid) {
+                load3(r, g.npad, s, acc);
+#pragma unroll
+                for (int e = 0; e < 9; e++) inv[e] = __ldg(op.dinv + e * np + s);
+            }
+        }
+    };
+    load(0);
+    for (int w = 0; w < 4 * per; w++) {
+        if (!sums) {
+            if (inplane && w % per == 0) row.load_x<true>(x, g.npad);
+            row.dots(wid, lane, dots[w & 1]);
+            if (w + 1 < 4 * per) load(w + 1);
+        }
+        __syncthreads();   // the table is complete; the other one has been read
+        if (sums) {
+            if (p >= 0) {
+#pragma unroll
+                for (int b = 0; b < 26; b++)
+#pragma unroll
+                    for (int e = 0; e < 3; e++) acc[e] -= dots[w & 1][b][e][lane];
+                x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
+                x[p + np] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
+                x[p + 2 * np] = dot3(inv[6], acc[0], inv[7], acc[1], inv[8], acc[2]);
+            }
+            if (w + 1 < 4 * per) load(w + 1);
+        }
+        if ((w + 1) % per == 0 && w + 1 < 4 * per) {   // the plane's next colour reads these values
+            if (cl > 1) cluster_barrier();
+            else __syncthreads();
+        }
+    }
+}
+
+// res = r - A x over every slot (unused slots get 0), 32 consecutive slots of
+// a colour at a time; NORM: the CTA's sum of |r - A x|^2 to partial.
+template <bool NORM>
+__global__ void __launch_bounds__(kThreads32)
+    residual_dense32_kernel(Geom g, DenseOp<float> op, const float *__restrict__ r, const float *__restrict__ x,
+                            float *__restrict__ res, double *__restrict__ partial) {
+    __shared__ DotTable dots[2];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const bool sums = wid == kDotWarps;
+    const size_t np = (size_t)g.npad;
+    const int items = 8 * ((g.S + 31) / 32);
+    BlockPair row;
+    float acc[3], cen[9], v[3];
+    int p = -1;
+    bool valid = false;
+    double sq = 0.0;
+    auto load = [&](int w) {
+        const int q = w & 7, t = 32 * (w >> 3) + lane;
+        const int I = t % g.M2, J = (t / g.M2) % g.N2, K = t / (g.M2 * g.N2);
+        valid = t < g.S && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n && 2 * K + (q >> 2) < g.o;
+        const int s = q * g.S + t;
+        if (!sums) {
+            row.load(op, g, valid, wid, I, J, K, q, s);
+            row.load_x<false>(x, g.npad);
+        } else {
+            p = t < g.S ? s : -1;
+            if (valid) {
+                load3(r, g.npad, s, acc);
+                load3(x, g.npad, s, v);
+#pragma unroll
+                for (int e = 0; e < 9; e++) cen[e] = __ldg(op.coef + (117 + e) * np + s);
+            }
+        }
+    };
+    int buf = 0;
+    if ((int)blockIdx.x < items) load(blockIdx.x);
+    for (int w = blockIdx.x; w < items; w += gridDim.x, buf ^= 1) {
+        const int next = w + gridDim.x;
+        if (!sums) {
+            row.dots(wid, lane, dots[buf]);
+            if (next < items) load(next);
+        }
+        __syncthreads();
+        if (sums) {
+            if (valid) {
+#pragma unroll
+                for (int b = 0; b < 13; b++)
+#pragma unroll
+                    for (int e = 0; e < 3; e++) acc[e] -= dots[buf][b][e][lane];
+                matvec_sub(cen, v, acc);
+#pragma unroll
+                for (int b = 13; b < 26; b++)
+#pragma unroll
+                    for (int e = 0; e < 3; e++) acc[e] -= dots[buf][b][e][lane];
+                if (NORM)
+                    sq += (double)acc[0] * (double)acc[0] + (double)acc[1] * (double)acc[1] +
+                          (double)acc[2] * (double)acc[2];
+            }
+            if (res && p >= 0) {
+#pragma unroll
+                for (int e = 0; e < 3; e++) res[p + e * np] = valid ? acc[e] : 0.0f;
+            }
+            if (next < items) load(next);
+        }
+    }
+    if (NORM && sums) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+        if (lane == 0) partial[blockIdx.x] = sq;
+    }
+}
+
+// ---------------------------------------------------------------- FP64
+constexpr int kNodes64 = 10;    // nodes of a team's item: lane 10 row + node
+constexpr int kTeams = 4;
+constexpr int kThreads64 = 128 * kTeams;
+
+// The blocks of one part for one (node, row) per lane.
+struct RowPart {
+    double a[kPartBlocks][3], v[kPartBlocks][3];
+    int s[kPartBlocks];
+
+    __device__ __forceinline__ void load(const DenseOp<double> &op, const Geom &g, bool valid, bool centre, int part,
+                                         int row, int I, int J, int K, int q, int p) {
+#pragma unroll
+        for (int u = 0; u < kPartBlocks; u++) {
+            const int b = part * kPartBlocks + u;
+            s[u] = valid && b < 27 && (centre || b != 13) ? block_slot(g, I, J, K, q, b) : -1;
+            const double *cb = op.coef + (size_t)(9 * b + 3 * row) * g.npad + p;
+#pragma unroll
+            for (int e = 0; e < 3; e++) a[u][e] = s[u] >= 0 ? __ldg(cb + (size_t)e * g.npad) : 0.0;
+        }
+    }
+    // x of the neighbours: of the node's own plane, of the other two, or all
+    template <bool COH, bool OWN, bool OTHER>
+    __device__ __forceinline__ void load_x(const double *x, int npad, int part) {
+#pragma unroll
+        for (int u = 0; u < kPartBlocks; u++) {
+            const int b = part * kPartBlocks + u;
+            const bool own = b >= 9 && b < 18;
+            if (own ? !OWN : !OTHER) continue;
+            if (s[u] >= 0) load3<double, COH>(x, npad, s[u], v[u]);
+            else v[u][0] = v[u][1] = v[u][2] = 0.0;
+        }
+    }
+    __device__ __forceinline__ double sum() const {
+        double t = 0.0;
+#pragma unroll
+        for (int u = 0; u < kPartBlocks; u++)
+#pragma unroll
+            for (int e = 0; e < 3; e++) t = fma_rn(a[u][e], v[u][e], t);
+        return t;
+    }
+};
+
+__device__ __forceinline__ void team_barrier(int team) {
+    asm volatile("bar.sync %0, 128;" ::"r"(team + 1) : "memory");
+}
+
+// The lane's row of a 3x3 matrix times the three rows of its node.
+__device__ __forceinline__ double row_times(const double (&m)[3], double acc, int node) {
+    const double a0 = __shfl_sync(0xffffffffu, acc, node), a1 = __shfl_sync(0xffffffffu, acc, node + kNodes64),
+                 a2 = __shfl_sync(0xffffffffu, acc, node + 2 * kNodes64);
+    return dot3(m[0], a0, m[1], a1, m[2], a2);
+}
+
+__global__ void __launch_bounds__(kThreads64)
+    gs_dense64_kernel(Geom g, int c, int cl, DenseOp<double> op, const double *__restrict__ r, double *x) {
+    __shared__ double parts[kTeams][2][4][32];
+    const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) & 3, team = threadIdx.x >> 7;
+    const int row = lane / kNodes64, node = lane - kNodes64 * row;   // row 3: two idle lanes
+    const int rank = blockIdx.x % cl, K = blockIdx.x / cl;
+    const int plane = g.M2 * g.N2, groups = (plane + kNodes64 - 1) / kNodes64;
+    const int per = (groups + cl * kTeams - 1) / (cl * kTeams);
+    const size_t np = (size_t)g.npad;
+    RowPart rp;
+    double acc = 0.0, inv[3] = {0.0, 0.0, 0.0};
+    int p = -1;
+    bool any = false;   // the item has a node: an empty one must not take the FP64 pipe from the others
+    // item w: the (w % per)-th 10 nodes of this team in colour w / per of the plane
+    auto load = [&](int w) {
+        const int q = 4 * c + w / per, t = kNodes64 * (rank + cl * (team + kTeams * (w % per))) + node;
+        const int J = t / g.M2, I = t - J * g.M2;
+        const bool valid = row < 3 && t < plane && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n;
+        const int s = q * g.S + K * plane + t;
+        any = __any_sync(0xffffffffu, valid);
+        if (!any) return;
+        rp.load(op, g, valid, false, part, row, I, J, K, q, s);
+        if (w % per != 0) rp.load_x<true, true, true>(x, g.npad, part);
+        else rp.load_x<true, false, true>(x, g.npad, part);
+        p = valid ? s : -1;
+        if (valid && (w & 3) == part) {   // this warp sums the item
+            acc = r[s + row * np];
+#pragma unroll
+            for (int e = 0; e < 3; e++) inv[e] = __ldg(op.dinv + (3 * row + e) * np + s);
+        }
+    };
+    load(0);
+    for (int w = 0; w < 4 * per; w++) {
+        if (any) {   // the same for the whole team
+            if (w % per == 0) rp.load_x<true, true, false>(x, g.npad, part);
+            parts[team][w & 1][part][lane] = rp.sum();
+            team_barrier(team);   // the item's parts are complete; the item before has been summed
+            if ((w & 3) == part) {
+#pragma unroll
+                for (int d = 0; d < 4; d++) acc -= parts[team][w & 1][d][lane];
+                const double xn = row_times(inv, acc, node);
+                if (p >= 0) x[p + row * np] = xn;
+            }
+        }
+        if (w + 1 < 4 * per) {
+            load(w + 1);
+            if ((w + 1) % per == 0) {   // the plane's next colour reads these values
+                if (cl > 1) cluster_barrier();
+                else __syncthreads();
+            }
+        }
+    }
+}
+
+template <typename R, bool NORM>
+__global__ void __launch_bounds__(kThreads64)
+    residual_dense64_kernel(Geom g, DenseOp<double> op, const double *__restrict__ r, const double *__restrict__ x,
+                            R *__restrict__ res, double *__restrict__ partial) {
+    __shared__ double parts[kTeams][2][4][32];
+    __shared__ double red[kThreads64 / 32];
+    const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) & 3, team = threadIdx.x >> 7;
+    const int row = lane / kNodes64, node = lane - kNodes64 * row;
+    const size_t np = (size_t)g.npad;
+    const int items = 8 * ((g.S + kNodes64 - 1) / kNodes64);
+    RowPart rp;
+    double acc = 0.0, sq = 0.0;
+    int p = -1;
+    bool valid = false;
+    auto load = [&](int w, int turn) {
+        const int q = w & 7, t = kNodes64 * (w >> 3) + node;
+        const int I = t % g.M2, J = (t / g.M2) % g.N2, K = t / (g.M2 * g.N2);
+        valid = row < 3 && t < g.S && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n && 2 * K + (q >> 2) < g.o;
+        const int s = q * g.S + t;
+        rp.load(op, g, valid, true, part, row, I, J, K, q, s);
+        rp.load_x<false, true, true>(x, g.npad, part);
+        p = row < 3 && t < g.S ? s : -1;
+        acc = valid && turn == part ? r[s + row * np] : 0.0;
+    };
+    const int step = gridDim.x * kTeams;
+    int turn = 0;
+    if ((int)(blockIdx.x * kTeams) + team < items) load(blockIdx.x * kTeams + team, 0);
+    for (int w = blockIdx.x * kTeams + team, n = 0; w < items; w += step, n++) {
+        parts[team][n & 1][part][lane] = rp.sum();
+        team_barrier(team);
+        if (turn == part) {
+            if (valid) {
+#pragma unroll
+                for (int d = 0; d < 4; d++) acc -= parts[team][n & 1][d][lane];
+                if (NORM) sq = fma_rn(acc, acc, sq);
+            }
+            if (res && p >= 0) res[p + row * np] = (R)acc;
+        }
+        turn = (turn + 1) & 3;
+        if (w + step < items) load(w + step, turn);
+    }
+    if (NORM) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+        if (lane == 0) red[threadIdx.x >> 5] = sq;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kThreads64 / 32; w++) sq += red[w];
+            partial[blockIdx.x] = sq;
+        }
+    }
+}
+
+// Launches one parity of planes, `cl` CTAs (one cluster) per plane.
+template <typename T, typename K>
+void launch_planes(K kernel, int threads, int cl, int planes, const Geom &g, int c, const DenseOp<T> &op, const T *r,
+                   T *x, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cl * planes);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cl;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, g, c, cl, op, r, x);
+}
+
+}  // namespace
+
+// One sweep of a level with per-node rows, two launches; the z extent is not
+// odd and periodic (a colour would then meet itself across the wrap).  The
+// cluster is as wide as a colour of the plane has groups of nodes, 8 CTAs at
+// most.
+template <typename T>
+void launch_gs_sweep_dense(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cudaStream_t st) {
+    const int nodes = sizeof(T) == 4 ? 32 : kNodes64, groups = (g.M2 * g.N2 + nodes - 1) / nodes;
+    const int cl = groups >= 8 ? 8 : groups >= 4 ? 4 : groups >= 2 ? 2 : 1;
+    for (int c = 0; c < 2; c++) {
+        const int planes = c == 0 ? (g.o + 1) / 2 : g.o / 2;
+        if (planes == 0) continue;
+        if constexpr (sizeof(T) == 4) launch_planes(gs_dense32_kernel, kThreads32, cl, planes, g, c, op.dop, r, x, st);
+        else launch_planes(gs_dense64_kernel, kThreads64, cl, planes, g, c, op.dop, r, x, st);
+    }
+}
+
+// res = r - A x of a level with per-node rows (res may be null); with partial
+// non-null, per-CTA sums of |r - A x|^2.  Returns the number of CTAs, at most
+// residual_blocks(g).
+template <typename T, typename R>
+int launch_residual_dense(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, R *res, double *partial,
+                          cudaStream_t st) {
+    // every CTA walks the slots: two an SM in FP32, one in FP64
+    if constexpr (sizeof(T) == 4) {
+        int grid = std::min(8 * ((g.S + 31) / 32), 2 * 152);
+        if (partial) grid = std::min(grid, residual_blocks(g));
+        if (partial) residual_dense32_kernel<true><<<grid, kThreads32, 0, st>>>(g, op.dop, r, x, res, partial);
+        else residual_dense32_kernel<false><<<grid, kThreads32, 0, st>>>(g, op.dop, r, x, res, nullptr);
+        return grid;
+    } else {
+        const int items = 8 * ((g.S + kNodes64 - 1) / kNodes64);
+        int grid = std::min((items + kTeams - 1) / kTeams, 152);
+        if (partial) grid = std::min(grid, residual_blocks(g));
+        if (partial) residual_dense64_kernel<R, true><<<grid, kThreads64, 0, st>>>(g, op.dop, r, x, res, partial);
+        else residual_dense64_kernel<R, false><<<grid, kThreads64, 0, st>>>(g, op.dop, r, x, res, nullptr);
+        return grid;
+    }
+}
+
+template void launch_gs_sweep_dense<float>(const LevelOp<float> &, const Geom &, const float *, float *, cudaStream_t);
+template void launch_gs_sweep_dense<double>(const LevelOp<double> &, const Geom &, const double *, double *,
+                                            cudaStream_t);
+template int launch_residual_dense<float, float>(const LevelOp<float> &, const Geom &, const float *, const float *,
+                                                 float *, double *, cudaStream_t);
+template int launch_residual_dense<double, double>(const LevelOp<double> &, const Geom &, const double *,
+                                                   const double *, double *, double *, cudaStream_t);
+template int launch_residual_dense<double, float>(const LevelOp<double> &, const Geom &, const double *,
+                                                  const double *, float *, double *, cudaStream_t);
+
+}  // namespace stzmg

@@ -28,6 +28,13 @@ void launch_gs_sweep(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cuda
 // use the tiled two-buffer sweep of tile.cu, with the same result
 template <typename T>
 void launch_gs_sweeps(const LevelOp<T> &op, const Geom &g, const T *r, T *x, T *tmp, int sweeps, cudaStream_t st);
+// dense.cu: one sweep in place, and the residual, of a level with per-node
+// rows (OP_DENSE); the residual returns its number of norm partials
+template <typename T>
+void launch_gs_sweep_dense(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cudaStream_t st);
+template <typename T, typename R>
+int launch_residual_dense(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, R *res, double *partial,
+                          cudaStream_t st);
 // tile.cu: one sweep reading xin and writing xout (levels periodic in x, y
 // with whole 32x32 tiles, shared-stencil or plane-invariant operators)
 template <typename T>
@@ -54,8 +61,8 @@ template <typename T>
 bool launch_residual_restrict(const LevelOp<T> &op, const Geom &g, const Geom &gc, const T *r, const T *x, T *rc,
                               cudaStream_t st);
 // How launch_gs_sweeps smooths a level: 0 eight colour launches per sweep,
-// 1 the tiled two-buffer sweep, 2 the band sweep, 3 the plane-phase kernels
-// (two launches per sweep each but the first)
+// 1 the tiled two-buffer sweep, 2 the band sweep, 3 the kernels that run the
+// four colours of a plane (two launches per sweep each but the first)
 template <typename T>
 int gs_sweep_kind(const LevelOp<T> &op, const Geom &g, const T *x, bool has_tmp);
 // 1 if a band CTA gave up waiting for its copies since the last call, 2 if

@@ -181,21 +181,41 @@ __device__ inline T lame_fix(const LameOp<T> &op, int p) {
 }
 
 // ---------------------------------------------------------------- dense
+// FP32: acc -= the block's three products, block by block.  FP64, whose pipe
+// issues one instruction per 64 cycles: the blocks' products accumulate with
+// fused multiply-adds in four parts, blocks 7 d .. 7 d + 6, which dense.cu
+// gives to the four schedulers of an SM; acc -= each part's sum in turn.
+constexpr int kPartBlocks = 7;
+
 template <typename T, bool WITH_CENTRE, bool COH = false>
 __device__ inline void dense_row(const DenseOp<T> &op, const Geom &g, const NbrOffsets &t, int p,
                                  const T *__restrict__ x, T *acc) {
     const size_t np = (size_t)g.npad;
+    T part[3] = {T(0), T(0), T(0)};
 #pragma unroll
     for (int b = 0; b < 27; b++) {
-        if (b == 13 && !WITH_CENTRE) continue;
         int s = t.ox[bdx(b) + 1] + t.oy[bdy(b) + 1] + t.oz[bdz(b) + 1];
-        if (s < 0) continue;   // outside a non-periodic grid: coefficients are zero there
-        T v[3], a[9];
-        load3<T, COH>(x, g.npad, s, v);
-        const T *cb = op.coef + (size_t)(9 * b) * np + p;
+        // outside a non-periodic grid: coefficients are zero there
+        if (!(b == 13 && !WITH_CENTRE) && s >= 0) {
+            T v[3], a[9];
+            load3<T, COH>(x, g.npad, s, v);
+            const T *cb = op.coef + (size_t)(9 * b) * np + p;
 #pragma unroll
-        for (int e = 0; e < 9; e++) a[e] = __ldg(cb + (size_t)e * np);
-        matvec_sub(a, v, acc);
+            for (int e = 0; e < 9; e++) a[e] = __ldg(cb + (size_t)e * np);
+            if (sizeof(T) == 4) {
+                matvec_sub(a, v, acc);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 9; e++) part[e / 3] = fma_rn(a[e], v[e % 3], part[e / 3]);
+            }
+        }
+        if (sizeof(T) == 8 && (b % kPartBlocks == kPartBlocks - 1 || b == 26)) {
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                acc[r] -= part[r];
+                part[r] = T(0);
+            }
+        }
     }
 }
 

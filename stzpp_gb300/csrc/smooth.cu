@@ -152,15 +152,10 @@ __device__ inline void gs_node(const LevelOp<T> &op, const Geom &g, int q, int I
         x[p + g.npad] = acc[1] / c3[1];
         x[p + 2 * g.npad] = acc[2] / c3[2];
         return;
-    } else if (KIND == OP_PLANE) {
+    } else {
         plane_row_coef<T, SPARSE, false>(cf, 1, g, nb, x, acc);
 #pragma unroll
         for (int e = 0; e < 9; e++) inv[e] = cf[243 + e];
-    } else {
-        dense_row<T, false>(op.dop, g, nb, p, x, acc);
-        const size_t np = (size_t)g.npad;
-#pragma unroll
-        for (int e = 0; e < 9; e++) inv[e] = __ldg(op.dop.dinv + (size_t)e * np + p);
     }
     x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
     x[p + g.npad] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
@@ -225,7 +220,7 @@ __device__ inline void block_sum_sq(double v, double *partial) {
 // residual before rounding to R) to partial[blockIdx.x].
 template <typename T, typename R, int KIND, bool ELASTIC, bool NORM>
 __global__ void __launch_bounds__(kBlock) residual_kernel(Geom g, const __grid_constant__ ConstOp<T> cop, LameOp<T> lop,
-                                                          DenseOp<T> dop, PlaneOp<T> pop, const T *__restrict__ r,
+                                                          PlaneOp<T> pop, const T *__restrict__ r,
                                                           const T *__restrict__ x, R *__restrict__ res,
                                                           double *__restrict__ partial) {
     // block (32, 8): lanes run along x, threadIdx.y is the colour, so a block
@@ -240,10 +235,7 @@ __global__ void __launch_bounds__(kBlock) residual_kernel(Geom g, const __grid_c
         T acc[3] = {T(0), T(0), T(0)};
         if (i < g.m && j < g.n && k < g.o) {
             load3(r, g.npad, p, acc);
-            if (KIND == OP_DENSE) {
-                NbrOffsets nb = nbr_offsets_sub(g, I, J, K, a, b, c);
-                dense_row<T, true>(dop, g, nb, p, x, acc);
-            } else if (KIND == OP_PLANE) {
+            if (KIND == OP_PLANE) {
                 NbrOffsets nb = nbr_offsets_sub(g, I, J, K, a, b, c);
                 if (pop.sparse) plane_row_coef<T, true, true>(pop.coef + k, pop.O, g, nb, x, acc);
                 else plane_row_coef<T, false, true>(pop.coef + k, pop.O, g, nb, x, acc);
@@ -326,10 +318,13 @@ void launch_gs_colour(const LevelOp<T> &op, const Geom &g, int q, const T *r, T 
 // the plane-phase kernels (one block per plane) pay off where a colour of a
 // plane is at most two nodes per thread, i.e. where launch latency dominates.
 // (An odd periodic z would put both parities of a colour on one plane.)
+static bool odd_periodic_z(const Geom &g) { return g.zp && (g.o & 1) && g.o > 1; }
+
 template <typename T>
-static bool large_planes(const Geom &g) {
+static bool large_planes(const LevelOp<T> &op, const Geom &g) {
+    if (op.kind == OP_DENSE) return odd_periodic_z(g);   // dense.cu takes planes of any size
     const int phase_max = sizeof(T) == 8 ? 256 : 2 * kPhaseThreads;   // FP64 needs every SM's FP64 units
-    return (g.zp && (g.o & 1) && g.o > 1) || g.M2 * g.N2 > phase_max;
+    return odd_periodic_z(g) || g.M2 * g.N2 > phase_max;
 }
 
 template <typename T>
@@ -348,7 +343,7 @@ void launch_gs_sweeps(const LevelOp<T> &op, const Geom &g, const T *r, T *x, T *
             launch_gs_sweep_band(op, g, r, tmp, x, st);
         }
     }
-    if (tmp && (large_planes<T>(g) || plane_tiles) && gs_tile_applies(op, g))
+    if (tmp && (large_planes(op, g) || plane_tiles) && gs_tile_applies(op, g))
         for (; s + 2 <= sweeps; s += 2) {
             launch_gs_sweep_tile(op, g, r, x, tmp, st);
             launch_gs_sweep_tile(op, g, r, tmp, x, st);
@@ -360,13 +355,13 @@ template <typename T>
 int gs_sweep_kind(const LevelOp<T> &op, const Geom &g, const T *x, bool has_tmp) {
     const bool plane_tiles = op.kind == OP_PLANE && g.m * g.n >= 64 * 64;
     if (has_tmp && gs_band_applies(op, g) && gs_band_ready(g, x)) return 2;
-    if (has_tmp && (large_planes<T>(g) || plane_tiles) && gs_tile_applies(op, g)) return 1;
-    return large_planes<T>(g) ? 0 : 3;
+    if (has_tmp && (large_planes(op, g) || plane_tiles) && gs_tile_applies(op, g)) return 1;
+    return large_planes(op, g) ? 0 : 3;
 }
 
 template <typename T>
 void launch_gs_sweep(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cudaStream_t st) {
-    if (large_planes<T>(g)) {
+    if (large_planes(op, g)) {
         for (int q = 0; q < 8; q++) launch_gs_colour(op, g, q, r, x, st);
         return;
     }
@@ -380,7 +375,7 @@ void launch_gs_sweep(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cuda
             if (op.pop.sparse) launch_phases<T, OP_PLANE, false, true>(op, g, r, x, st);
             else launch_phases<T, OP_PLANE, false, false>(op, g, r, x, st);
             break;
-        default: launch_phases<T, OP_DENSE, false, false>(op, g, r, x, st); break;
+        default: launch_gs_sweep_dense<T>(op, g, r, x, st); break;
     }
 }
 
@@ -393,18 +388,15 @@ static void launch_residual_k(const LevelOp<T> &op, const Geom &g, const T *r, c
     switch (op.kind) {
         case OP_CONST:
             if (op.cop.elastic)
-                residual_kernel<T, R, OP_CONST, true, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.dop, op.pop, r, x, res, partial);
+                residual_kernel<T, R, OP_CONST, true, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.pop, r, x, res, partial);
             else
-                residual_kernel<T, R, OP_CONST, false, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.dop, op.pop, r, x, res, partial);
+                residual_kernel<T, R, OP_CONST, false, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.pop, r, x, res, partial);
             break;
         case OP_LAME:
-            residual_kernel<T, R, OP_LAME, false, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.dop, op.pop, r, x, res, partial);
-            break;
-        case OP_PLANE:
-            residual_kernel<T, R, OP_PLANE, false, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.dop, op.pop, r, x, res, partial);
+            residual_kernel<T, R, OP_LAME, false, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.pop, r, x, res, partial);
             break;
         default:
-            residual_kernel<T, R, OP_DENSE, false, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.dop, op.pop, r, x, res, partial);
+            residual_kernel<T, R, OP_PLANE, false, NORM><<<blocks, blk, 0, st>>>(g, op.cop, op.lop, op.pop, r, x, res, partial);
             break;
     }
 }
@@ -420,6 +412,11 @@ void launch_residual(const LevelOp<T> &op, const Geom &g, const T *r, const T *x
     if (std::is_same<T, R>::value && res && residual_tile_applies(op, g)) {
         launch_residual_tile<T>(op, g, r, x, reinterpret_cast<T *>(res), partial, st);
         if (partial && out) sum_partials_kernel<<<1, 1024, 0, st>>>(partial, residual_tile_blocks(g, sizeof(T) == 8), out);
+        return;
+    }
+    if (op.kind == OP_DENSE) {
+        const int nb = launch_residual_dense<T, R>(op, g, r, x, res, partial, st);
+        if (partial && out) sum_partials_kernel<<<1, 1024, 0, st>>>(partial, nb, out);
         return;
     }
     if (partial) launch_residual_k<T, R, true>(op, g, r, x, res, partial, st);
