@@ -72,7 +72,7 @@ struct ApiError {
 template <typename T>
 struct Level {
     T *x = nullptr, *r = nullptr, *res = nullptr;   // 3*npad each
-    T *coef = nullptr, *dinv = nullptr;             // coarse operators (243 and 9 per row)
+    T *coef = nullptr, *dinv = nullptr;             // coarse operators (243 and 9 values per row)
     size_t coef_rows = 0;                           // rows coef / dinv were allocated for
 };
 
@@ -278,7 +278,7 @@ void alloc_fields(stz_mg_handle h) {
         }
     }
     h->partial_len = residual_blocks(h->geo[0]);
-    h->partial = h->alloc<double>(h->partial_len);
+    h->partial = h->alloc<double>(std::max(h->partial_len, kDensePartials));
     h->dscal = h->alloc<double>(8);
     h->dflag = h->alloc<int>(4);
     CK(cudaMallocHost(&h->hscal, 8 * sizeof(double)));
@@ -563,7 +563,7 @@ void build_bottom(stz_mg_handle h) {
     {
         const double *src = nullptr;
         if (h->op64[lb].kind != OP_DENSE) {
-            h->ensure(h->bot_dense, h->bot_dense_len, 243 * (size_t)g.npad);
+            h->ensure(h->bot_dense, h->bot_dense_len, coef_len(g.npad));
             launch_expand_dense(h->op64[lb], g, h->bot_dense, h->st);
             src = h->bot_dense;
         } else {
@@ -721,8 +721,8 @@ void setup(stz_mg_handle h) {
         check_launch();
         h->op64[0].dop.dinv = h->top_dinv64;
         if (mixed) {
-            launch_convert(h->top_coef64, h->top_coef32, 243 * (size_t)g.npad, h->st);
-            launch_convert(h->top_dinv64, h->top_dinv32, 9 * (size_t)g.npad, h->st);
+            launch_convert(h->top_coef64, h->top_coef32, coef_len(g.npad), h->st);
+            launch_convert(h->top_dinv64, h->top_dinv32, dinv_len(g.npad), h->st);
             check_launch();
             h->op32[0].dop.coef = h->top_coef32;
             h->op32[0].dop.dinv = h->top_dinv32;
@@ -738,12 +738,13 @@ void setup(stz_mg_handle h) {
     for (int l = 1; l < h->nlev; l++) {
         const Geom &gf = h->geo[l - 1], &gc = h->geo[l];
         const size_t rows = plane ? (size_t)gc.o : (size_t)gc.npad;
+        const size_t ncoef = plane ? 243 * rows : coef_len(rows), ndinv = plane ? 9 * rows : dinv_len(rows);
         Level<double> &C = h->L64[l];
         if (C.coef_rows != rows) {
             h->release(C.coef);
             h->release(C.dinv);
-            C.coef = h->alloc<double>(243 * rows);
-            C.dinv = h->alloc<double>(9 * rows);
+            C.coef = h->alloc<double>(ncoef);
+            C.dinv = h->alloc<double>(ndinv);
             C.coef_rows = rows;
         }
         launch_rat_bounds(gf, h->S[l - 1], gc, h->S[l], h->dflag + 1, h->st);
@@ -790,12 +791,12 @@ void setup(stz_mg_handle h) {
             if (F.coef_rows != rows) {
                 h->release(F.coef);
                 h->release(F.dinv);
-                F.coef = h->alloc<float>(243 * rows);
-                F.dinv = h->alloc<float>(9 * rows);
+                F.coef = h->alloc<float>(ncoef);
+                F.dinv = h->alloc<float>(ndinv);
                 F.coef_rows = rows;
             }
-            launch_convert(C.coef, F.coef, 243 * rows, h->st);
-            launch_convert(C.dinv, F.dinv, 9 * rows, h->st);
+            launch_convert(C.coef, F.coef, ncoef, h->st);
+            launch_convert(C.dinv, F.dinv, ndinv, h->st);
             check_launch();
             h->op32[l] = LevelOp<float>{};
             if (plane) {
@@ -1168,14 +1169,14 @@ int stz_mg_set_stencil_points(stz_mg_handle h, const double *A, int where) {
         const double *src = to_device(h, A, n, where);
         require_finite(h, src, n, "stencil");
         if (!h->top_coef64) {
-            h->top_coef64 = h->alloc<double>(243 * (size_t)g.npad);
-            h->top_dinv64 = h->alloc<double>(9 * (size_t)g.npad);
+            h->top_coef64 = h->alloc<double>(coef_len(g.npad));
+            h->top_dinv64 = h->alloc<double>(dinv_len(g.npad));
             if (h->d.precision == STZ_MG_MIXED) {
-                h->top_coef32 = h->alloc<float>(243 * (size_t)g.npad);
-                h->top_dinv32 = h->alloc<float>(9 * (size_t)g.npad);
+                h->top_coef32 = h->alloc<float>(coef_len(g.npad));
+                h->top_dinv32 = h->alloc<float>(dinv_len(g.npad));
             }
         }
-        CK(cudaMemsetAsync(h->top_coef64, 0, 243 * (size_t)g.npad * sizeof(double), h->st));
+        CK(cudaMemsetAsync(h->top_coef64, 0, coef_len(g.npad) * sizeof(double), h->st));
         launch_coef_nat_to_cb(g, src, h->top_coef64, h->st);
         check_launch();
         // Dirichlet nodes keep only their centre block (fill_entries stores one entry)
@@ -1511,7 +1512,7 @@ int stz_mg_level_operator(stz_mg_handle h, int level, double *A, int *S) {
             double *dcoef = nullptr;
             const double *src;
             if (h->op64[level].kind != OP_DENSE) {
-                dcoef = h->alloc<double>(243 * (size_t)g.npad);
+                dcoef = h->alloc<double>(coef_len(g.npad));
                 launch_expand_dense(h->op64[level], g, dcoef, h->st);
                 src = dcoef;
             } else {

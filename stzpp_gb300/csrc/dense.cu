@@ -26,10 +26,10 @@
 //
 // One sweep on GB300, before (one block a plane on planes of up to 64x64,
 // else eight colour launches, a thread a node) and now:
-//   64x64x65  FP32  310 -> 97 us     16x16x17  FP32   54 -> 20 us
-//   49x41x33  FP64  328 -> 180 us    32x48x26  FP64  245 -> 84 us
-//   7x6x5     FP64  118 -> 38 us
-// and the residual of 49x41x33 in FP64 72 -> 65 us, of 16x16x17 in FP32 23 -> 3 us.
+//   64x64x65  FP32  310 -> 69 us     16x16x17  FP32   54 -> 14 us
+//   49x41x33  FP64  328 -> 148 us    32x48x26  FP64  245 -> 66 us
+//   7x6x5     FP64  118 -> 31 us
+// and the residual of 49x41x33 in FP64 72 -> 59 us, of 16x16x17 in FP32 23 -> 3 us.
 #include <algorithm>
 
 #include "launch.h"
@@ -39,27 +39,44 @@ namespace stzmg {
 
 namespace {
 
-constexpr int kOut = INT32_MIN / 4;   // outside a non-periodic grid
+// Entry d + 1 of a dimension's neighbour offsets, d known at run time.
+__device__ __forceinline__ int pick(const int (&o)[3], int d) { return d == 0 ? o[1] : d < 0 ? o[0] : o[2]; }
 
-// Slot offset of the neighbour d of sub-grid coordinate I (parity a) along one
-// dimension: one entry of dim_offsets.
-__device__ __forceinline__ int dim_off(int I, int a, int n, int N2, int prd, int pstride, int istride, int d) {
-    const int own = a * pstride + I * istride;
-    if (d == 0) return own;
-    if (n == 1) return prd ? own : kOut;
-    if (d < 0) return a ? I * istride : I > 0 ? pstride + (I - 1) * istride : prd ? pstride + (N2 - 1) * istride : kOut;
-    return 2 * I + a + 1 < n ? (a ? (I + 1) * istride : pstride + I * istride) : prd ? 0 : kOut;
+// Offsets of the neighbours in the plane, of a node of colour q.
+__device__ __forceinline__ void plane_offsets(const Geom &g, int I, int J, int q, NbrOffsets &t) {
+    dim_offsets(I, q & 1, g.m, g.M2, g.xp, g.S, 1, t.ox);
+    dim_offsets(J, (q >> 1) & 1, g.n, g.N2, g.yp, 2 * g.S, g.M2, t.oy);
+}
+__device__ __forceinline__ void z_offsets(const Geom &g, int K, int q, NbrOffsets &t) {
+    dim_offsets(K, q >> 2, g.o, g.O2, g.zp, 4 * g.S, g.M2 * g.N2, t.oz);
 }
 
-// Slot of the neighbour through block b of node (I, J, K) of colour q; negative outside the grid.
-__device__ __forceinline__ int block_slot(const Geom &g, int I, int J, int K, int q, int b) {
-    return dim_off(I, q & 1, g.m, g.M2, g.xp, g.S, 1, b % 3 - 1) +
-           dim_off(J, (q >> 1) & 1, g.n, g.N2, g.yp, 2 * g.S, g.M2, (b / 3) % 3 - 1) +
-           dim_off(K, q >> 2, g.o, g.O2, g.zp, 4 * g.S, g.M2 * g.N2, b / 9 - 1);
-}
+// Sub-grid coordinates of a lane's node that moves on by a fixed number of
+// slots per item (no division per item).
+struct Walk {
+    int t, I, J, K;
+    int dt, dI, dJ, dK;
+    __device__ __forceinline__ Walk(const Geom &g, int t0, int step) : t(t0), dt(step) {
+        I = t0 % g.M2, J = t0 / g.M2 % g.N2, K = t0 / (g.M2 * g.N2);
+        dI = step % g.M2, dJ = step / g.M2 % g.N2, dK = step / (g.M2 * g.N2);
+    }
+    __device__ __forceinline__ void next(const Geom &g) {
+        t += dt;
+        I += dI, J += dJ, K += dK;
+        if (I >= g.M2) I -= g.M2, J++;
+        if (J >= g.N2) J -= g.N2, K++;
+    }
+};
 
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// The end of a colour.  A thread arrives when its own values are stored and
+// loads what the next colour needs and does not depend on this one before it
+// waits: a release waits for every load issued before it too.
+__device__ __forceinline__ void colour_arrive(int cl) {
+    if (cl > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void colour_wait(int cl) {
+    if (cl > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
 }
 
 // ---------------------------------------------------------------- FP32
@@ -68,36 +85,34 @@ constexpr int kThreads32 = 32 * (kDotWarps + 1);     // the last warp sums
 
 using DotTable = float[26][3][32];
 
-// What a dot warp holds of its two blocks for one node per lane.
+// What a dot warp holds of its blocks w and 26 - w for one node per lane
+// (coefficients of slot 0 for a lane without a node).
 struct BlockPair {
     float a[2][9], v[2][3];
-    int s[2];
+    int s[2];   // the neighbours' slots, negative outside the grid
 
-    // coefficients of blocks w and 26 - w at slot p, and the neighbours' slots
-    __device__ __forceinline__ void load(const DenseOp<float> &op, const Geom &g, bool valid, int w, int I, int J,
-                                         int K, int q, int p) {
+    __device__ __forceinline__ void load(const DenseOp<float> &op, int w, int p, const NbrOffsets &t, bool valid) {
+        const int dx = bdx(w), dy = bdy(w), dz = bdz(w);
+        s[0] = valid ? pick(t.ox, dx) + pick(t.oy, dy) + pick(t.oz, dz) : -1;
+        s[1] = valid ? pick(t.ox, -dx) + pick(t.oy, -dy) + pick(t.oz, -dz) : -1;
+        const float *row = op.coef + coef_at(p) + 9 * w * kCoefGroup, *row2 = row + 9 * (26 - 2 * w) * kCoefGroup;
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int b = u ? 26 - w : w;
-            s[u] = valid ? block_slot(g, I, J, K, q, b) : -1;
-            const float *cb = op.coef + (size_t)(9 * b) * g.npad + p;
-#pragma unroll
-            for (int e = 0; e < 9; e++) a[u][e] = s[u] >= 0 ? __ldg(cb + (size_t)e * g.npad) : 0.0f;
+        for (int e = 0; e < 9; e++) {
+            a[0][e] = __ldg(row + e * kCoefGroup);
+            a[1][e] = __ldg(row2 + e * kCoefGroup);
         }
     }
     template <bool COH>
     __device__ __forceinline__ void load_x(const float *x, int npad) {
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            if (s[u] >= 0) load3<float, COH>(x, npad, s[u], v[u]);
-            else v[u][0] = v[u][1] = v[u][2] = 0.0f;
-        }
+        for (int u = 0; u < 2; u++) load3<float, COH>(x, npad, max(s[u], 0), v[u]);
     }
     // the products, into the CTA's table (0 for a neighbour outside the grid)
-    __device__ __forceinline__ void dots(int w, int lane, DotTable &out) const {
+    __device__ __forceinline__ void dots(int w, int lane, DotTable &out) {
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             float(*o)[32] = out[u ? 25 - w : w];
+            if (s[u] < 0) v[u][0] = v[u][1] = v[u][2] = 0.0f;
 #pragma unroll
             for (int r = 0; r < 3; r++)
                 o[r][lane] = dot3(a[u][3 * r], v[u][0], a[u][3 * r + 1], v[u][1], a[u][3 * r + 2], v[u][2]);
@@ -107,7 +122,7 @@ struct BlockPair {
 
 // Colours 4c .. 4c+3 of every plane of parity c, `cl` CTAs (one cluster) per
 // plane; x is updated in place.
-__global__ void __launch_bounds__(kThreads32)
+__global__ void __launch_bounds__(kThreads32, 2)
     gs_dense32_kernel(Geom g, int c, int cl, DenseOp<float> op, const float *__restrict__ r, float *x) {
     __shared__ DotTable dots[2];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -116,96 +131,107 @@ __global__ void __launch_bounds__(kThreads32)
     const bool sums = wid == kDotWarps;
     const bool inplane = wid >= 9;   // blocks 9 .. 12 and 14 .. 17; the other warps read the planes above and below
     const size_t np = (size_t)g.npad;
+    const Walk start(g, 32 * rank + lane, 32 * cl);
+    Walk at = start;
     BlockPair row;
     float acc[3], inv[9];
     int p = -1;   // the summing warp's node
-    // item w: the (w % per)-th 32 nodes of this CTA in colour w / per of the plane
-    auto load = [&](int w) {
-        const int q = 4 * c + w / per, t = 32 * (rank + cl * (w % per)) + lane;
-        const int J = t / g.M2, I = t - J * g.M2;
-        const bool valid = t < plane && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n;
-        const int s = q * g.S + K * plane + t;
+    NbrOffsets nb;
+    z_offsets(g, K, 4 * c, nb);
+    // 32 nodes of colour q of the plane: all that may be read before the colour begins (first) or in it
+    auto load = [&](int q, bool first) {
+        const bool valid = at.t < plane && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n;
+        const int s = valid ? q * g.S + K * plane + at.t : 0;
         if (!sums) {
-            row.load(op, g, valid, wid, I, J, K, q, s);
-            // a colour's own plane is final once the colour before it is done
-            if (!inplane || w % per != 0) row.load_x<true>(x, g.npad);
+            plane_offsets(g, at.I, at.J, q, nb);
+            row.load(op, wid, s, nb, valid);
+            if (!inplane || !first) row.load_x<true>(x, g.npad);
         } else {
             p = valid ? s : -1;
-            if (valid) {
-                load3(r, g.npad, s, acc);
+            load3(r, g.npad, s, acc);
 #pragma unroll
-                for (int e = 0; e < 9; e++) inv[e] = __ldg(op.dinv + e * np + s);
-            }
+            for (int e = 0; e < 9; e++) inv[e] = __ldg(op.dinv + dinv_at(s) + e * kCoefGroup);
         }
     };
-    load(0);
-    for (int w = 0; w < 4 * per; w++) {
-        if (!sums) {
-            if (inplane && w % per == 0) row.load_x<true>(x, g.npad);
-            row.dots(wid, lane, dots[w & 1]);
-            if (w + 1 < 4 * per) load(w + 1);
-        }
-        __syncthreads();   // the table is complete; the other one has been read
-        if (sums) {
-            if (p >= 0) {
-#pragma unroll
-                for (int b = 0; b < 26; b++)
-#pragma unroll
-                    for (int e = 0; e < 3; e++) acc[e] -= dots[w & 1][b][e][lane];
-                x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
-                x[p + np] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
-                x[p + 2 * np] = dot3(inv[6], acc[0], inv[7], acc[1], inv[8], acc[2]);
+    int buf = 0;
+    load(4 * c, true);
+#pragma unroll 1
+    for (int q = 4 * c; q < 4 * c + 4; q++) {
+#pragma unroll 1
+        for (int n = 0; n < per; n++, buf ^= 1) {
+            const bool last = n + 1 == per;
+            if (last) at = start;
+            else at.next(g);
+            if (!sums) {
+                if (inplane && n == 0) row.load_x<true>(x, g.npad);
+                row.dots(wid, lane, dots[buf]);
+                if (!last) load(q, false);
             }
-            if (w + 1 < 4 * per) load(w + 1);
+            __syncthreads();   // the table is complete; the other one has been read
+            if (sums) {
+                if (p >= 0) {
+#pragma unroll
+                    for (int b = 0; b < 26; b++)
+#pragma unroll
+                        for (int e = 0; e < 3; e++) acc[e] -= dots[buf][b][e][lane];
+                    x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
+                    x[p + np] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
+                    x[p + 2 * np] = dot3(inv[6], acc[0], inv[7], acc[1], inv[8], acc[2]);
+                }
+                if (!last) load(q, false);
+            }
         }
-        if ((w + 1) % per == 0 && w + 1 < 4 * per) {   // the plane's next colour reads these values
-            if (cl > 1) cluster_barrier();
-            else __syncthreads();
+        if (q < 4 * c + 3) {   // the plane's next colour reads these values
+            colour_arrive(cl);
+            load(q + 1, true);
+            colour_wait(cl);
         }
     }
 }
 
 // res = r - A x over every slot (unused slots get 0), 32 consecutive slots of
-// a colour at a time; NORM: the CTA's sum of |r - A x|^2 to partial.
+// a colour at a time, colour blockIdx.x % 8; NORM: the CTA's sum of
+// |r - A x|^2 to partial.
 template <bool NORM>
 __global__ void __launch_bounds__(kThreads32)
     residual_dense32_kernel(Geom g, DenseOp<float> op, const float *__restrict__ r, const float *__restrict__ x,
                             float *__restrict__ res, double *__restrict__ partial) {
     __shared__ DotTable dots[2];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = blockIdx.x & 7;
     const bool sums = wid == kDotWarps;
     const size_t np = (size_t)g.npad;
-    const int items = 8 * ((g.S + 31) / 32);
+    const int t0 = 32 * (blockIdx.x >> 3), step = 32 * (gridDim.x >> 3);
+    Walk at(g, t0 + lane, step);
     BlockPair row;
     float acc[3], cen[9], v[3];
     int p = -1;
     bool valid = false;
     double sq = 0.0;
-    auto load = [&](int w) {
-        const int q = w & 7, t = 32 * (w >> 3) + lane;
-        const int I = t % g.M2, J = (t / g.M2) % g.N2, K = t / (g.M2 * g.N2);
-        valid = t < g.S && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n && 2 * K + (q >> 2) < g.o;
-        const int s = q * g.S + t;
+    auto load = [&]() {
+        valid = at.t < g.S && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n && 2 * at.K + (q >> 2) < g.o;
+        const int s = valid ? q * g.S + at.t : 0;
         if (!sums) {
-            row.load(op, g, valid, wid, I, J, K, q, s);
+            NbrOffsets nb;
+            plane_offsets(g, at.I, at.J, q, nb);
+            z_offsets(g, at.K, q, nb);
+            row.load(op, wid, s, nb, valid);
             row.load_x<false>(x, g.npad);
         } else {
-            p = t < g.S ? s : -1;
-            if (valid) {
-                load3(r, g.npad, s, acc);
-                load3(x, g.npad, s, v);
+            p = at.t < g.S ? q * g.S + at.t : -1;
+            load3(r, g.npad, s, acc);
+            load3(x, g.npad, s, v);
 #pragma unroll
-                for (int e = 0; e < 9; e++) cen[e] = __ldg(op.coef + (117 + e) * np + s);
-            }
+            for (int e = 0; e < 9; e++) cen[e] = __ldg(op.coef + coef_at(s) + (117 + e) * kCoefGroup);
         }
     };
+    if (t0 < g.S) load();
     int buf = 0;
-    if ((int)blockIdx.x < items) load(blockIdx.x);
-    for (int w = blockIdx.x; w < items; w += gridDim.x, buf ^= 1) {
-        const int next = w + gridDim.x;
+    for (int t = t0; t < g.S; t += step, buf ^= 1) {
+        const bool more = t + step < g.S;
         if (!sums) {
             row.dots(wid, lane, dots[buf]);
-            if (next < items) load(next);
+            at.next(g);
+            if (more) load();
         }
         __syncthreads();
         if (sums) {
@@ -227,7 +253,8 @@ __global__ void __launch_bounds__(kThreads32)
 #pragma unroll
                 for (int e = 0; e < 3; e++) res[p + e * np] = valid ? acc[e] : 0.0f;
             }
-            if (next < items) load(next);
+            at.next(g);
+            if (more) load();
         }
     }
     if (NORM && sums) {
@@ -242,21 +269,33 @@ constexpr int kNodes64 = 10;    // nodes of a team's item: lane 10 row + node
 constexpr int kTeams = 4;
 constexpr int kThreads64 = 128 * kTeams;
 
-// The blocks of one part for one (node, row) per lane.
+// The blocks of one part for one (node, row) per lane (coefficients of slot 0
+// for a lane without a node).
 struct RowPart {
     double a[kPartBlocks][3], v[kPartBlocks][3];
-    int s[kPartBlocks];
+    int s[kPartBlocks];   // the neighbours' slots, negative outside the grid
 
-    __device__ __forceinline__ void load(const DenseOp<double> &op, const Geom &g, bool valid, bool centre, int part,
-                                         int row, int I, int J, int K, int q, int p) {
+    template <int PART, bool CENTRE>
+    __device__ __forceinline__ void load_part(const DenseOp<double> &op, bool valid, int row, const NbrOffsets &t,
+                                              int p) {
+        const double *c = op.coef + coef_at(p) + 3 * row * kCoefGroup;
 #pragma unroll
         for (int u = 0; u < kPartBlocks; u++) {
-            const int b = part * kPartBlocks + u;
-            s[u] = valid && b < 27 && (centre || b != 13) ? block_slot(g, I, J, K, q, b) : -1;
-            const double *cb = op.coef + (size_t)(9 * b + 3 * row) * g.npad + p;
+            const int b = PART * kPartBlocks + u;
+            const bool here = b < 27 && (CENTRE || b != 13);
+            s[u] = here && valid ? t.ox[bdx(b) + 1] + t.oy[bdy(b) + 1] + t.oz[bdz(b) + 1] : -1;
 #pragma unroll
-            for (int e = 0; e < 3; e++) a[u][e] = s[u] >= 0 ? __ldg(cb + (size_t)e * g.npad) : 0.0;
+            for (int e = 0; e < 3; e++) a[u][e] = here ? __ldg(c + (9 * b + e) * kCoefGroup) : 0.0;
         }
+    }
+    // the block numbers have to be known when the kernel is compiled: the offsets then stay in registers
+    template <bool CENTRE>
+    __device__ __forceinline__ void load(const DenseOp<double> &op, bool valid, int part, int row, const NbrOffsets &t,
+                                         int p) {
+        if (part == 0) load_part<0, CENTRE>(op, valid, row, t, p);
+        else if (part == 1) load_part<1, CENTRE>(op, valid, row, t, p);
+        else if (part == 2) load_part<2, CENTRE>(op, valid, row, t, p);
+        else load_part<3, CENTRE>(op, valid, row, t, p);
     }
     // x of the neighbours: of the node's own plane, of the other two, or all
     template <bool COH, bool OWN, bool OTHER>
@@ -266,8 +305,8 @@ struct RowPart {
             const int b = part * kPartBlocks + u;
             const bool own = b >= 9 && b < 18;
             if (own ? !OWN : !OTHER) continue;
-            if (s[u] >= 0) load3<double, COH>(x, npad, s[u], v[u]);
-            else v[u][0] = v[u][1] = v[u][2] = 0.0;
+            load3<double, COH>(x, npad, max(s[u], 0), v[u]);
+            if (s[u] < 0) v[u][0] = v[u][1] = v[u][2] = 0.0;
         }
     }
     __device__ __forceinline__ double sum() const {
@@ -300,47 +339,60 @@ __global__ void __launch_bounds__(kThreads64)
     const int plane = g.M2 * g.N2, groups = (plane + kNodes64 - 1) / kNodes64;
     const int per = (groups + cl * kTeams - 1) / (cl * kTeams);
     const size_t np = (size_t)g.npad;
+    const Walk start(g, kNodes64 * (rank + cl * team) + node, kNodes64 * cl * kTeams);
+    Walk at = start;
     RowPart rp;
     double acc = 0.0, inv[3] = {0.0, 0.0, 0.0};
     int p = -1;
     bool any = false;   // the item has a node: an empty one must not take the FP64 pipe from the others
-    // item w: the (w % per)-th 10 nodes of this team in colour w / per of the plane
-    auto load = [&](int w) {
-        const int q = 4 * c + w / per, t = kNodes64 * (rank + cl * (team + kTeams * (w % per))) + node;
-        const int J = t / g.M2, I = t - J * g.M2;
-        const bool valid = row < 3 && t < plane && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n;
-        const int s = q * g.S + K * plane + t;
+    NbrOffsets nb;
+    z_offsets(g, K, 4 * c, nb);
+    // 10 nodes of colour q of the plane: all that may be read before the colour begins (first) or in it
+    auto load = [&](int q, bool first, bool mine) {
+        const bool valid =
+            row < 3 && at.t < plane && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n;
         any = __any_sync(0xffffffffu, valid);
         if (!any) return;
-        rp.load(op, g, valid, false, part, row, I, J, K, q, s);
-        if (w % per != 0) rp.load_x<true, true, true>(x, g.npad, part);
-        else rp.load_x<true, false, true>(x, g.npad, part);
+        const int s = valid ? q * g.S + K * plane + at.t : 0;
+        plane_offsets(g, at.I, at.J, q, nb);
+        rp.load<false>(op, valid, part, row < 3 ? row : 0, nb, s);
+        if (first) rp.load_x<true, false, true>(x, g.npad, part);
+        else rp.load_x<true, true, true>(x, g.npad, part);
         p = valid ? s : -1;
-        if (valid && (w & 3) == part) {   // this warp sums the item
+        if (valid && mine) {
             acc = r[s + row * np];
 #pragma unroll
-            for (int e = 0; e < 3; e++) inv[e] = __ldg(op.dinv + (3 * row + e) * np + s);
+            for (int e = 0; e < 3; e++) inv[e] = __ldg(op.dinv + dinv_at(s) + (3 * row + e) * kCoefGroup);
         }
     };
-    load(0);
-    for (int w = 0; w < 4 * per; w++) {
-        if (any) {   // the same for the whole team
-            if (w % per == 0) rp.load_x<true, true, false>(x, g.npad, part);
-            parts[team][w & 1][part][lane] = rp.sum();
-            team_barrier(team);   // the item's parts are complete; the item before has been summed
-            if ((w & 3) == part) {
+    int w = 0;   // items so far: the warps take turns at the sums
+    load(4 * c, true, part == 0);
+#pragma unroll 1
+    for (int q = 4 * c; q < 4 * c + 4; q++) {
+#pragma unroll 1
+        for (int n = 0; n < per; n++, w++) {
+            if (any) {   // the same for the whole team
+                if (n == 0) rp.load_x<true, true, false>(x, g.npad, part);
+                parts[team][w & 1][part][lane] = rp.sum();
+                team_barrier(team);   // the item's parts are complete; the item before has been summed
+                if ((w & 3) == part) {
 #pragma unroll
-                for (int d = 0; d < 4; d++) acc -= parts[team][w & 1][d][lane];
-                const double xn = row_times(inv, acc, node);
-                if (p >= 0) x[p + row * np] = xn;
+                    for (int d = 0; d < 4; d++) acc -= parts[team][w & 1][d][lane];
+                    const double xn = row_times(inv, acc, node);
+                    if (p >= 0) x[p + row * np] = xn;
+                }
+            }
+            if (n + 1 == per) {
+                at = start;
+            } else {
+                at.next(g);
+                load(q, false, ((w + 1) & 3) == part);
             }
         }
-        if (w + 1 < 4 * per) {
-            load(w + 1);
-            if ((w + 1) % per == 0) {   // the plane's next colour reads these values
-                if (cl > 1) cluster_barrier();
-                else __syncthreads();
-            }
+        if (q < 4 * c + 3) {   // the plane's next colour reads these values
+            colour_arrive(cl);
+            load(q + 1, true, (w & 3) == part);
+            colour_wait(cl);
         }
     }
 }
@@ -354,28 +406,30 @@ __global__ void __launch_bounds__(kThreads64)
     const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) & 3, team = threadIdx.x >> 7;
     const int row = lane / kNodes64, node = lane - kNodes64 * row;
     const size_t np = (size_t)g.npad;
-    const int items = 8 * ((g.S + kNodes64 - 1) / kNodes64);
+    const int q = blockIdx.x & 7;
+    const int t0 = kNodes64 * ((blockIdx.x >> 3) * kTeams + team), step = kNodes64 * (gridDim.x >> 3) * kTeams;
+    Walk at(g, t0 + node, step);
     RowPart rp;
     double acc = 0.0, sq = 0.0;
     int p = -1;
     bool valid = false;
-    auto load = [&](int w, int turn) {
-        const int q = w & 7, t = kNodes64 * (w >> 3) + node;
-        const int I = t % g.M2, J = (t / g.M2) % g.N2, K = t / (g.M2 * g.N2);
-        valid = row < 3 && t < g.S && 2 * I + (q & 1) < g.m && 2 * J + ((q >> 1) & 1) < g.n && 2 * K + (q >> 2) < g.o;
-        const int s = q * g.S + t;
-        rp.load(op, g, valid, true, part, row, I, J, K, q, s);
+    auto load = [&](bool mine) {
+        valid = row < 3 && at.t < g.S && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n &&
+                2 * at.K + (q >> 2) < g.o;
+        const int s = valid ? q * g.S + at.t : 0;
+        NbrOffsets nb;
+        plane_offsets(g, at.I, at.J, q, nb);
+        z_offsets(g, at.K, q, nb);
+        rp.load<true>(op, valid, part, row < 3 ? row : 0, nb, s);
         rp.load_x<false, true, true>(x, g.npad, part);
-        p = row < 3 && t < g.S ? s : -1;
-        acc = valid && turn == part ? r[s + row * np] : 0.0;
+        p = row < 3 && at.t < g.S ? q * g.S + at.t : -1;
+        acc = valid && mine ? r[s + row * np] : 0.0;
     };
-    const int step = gridDim.x * kTeams;
-    int turn = 0;
-    if ((int)(blockIdx.x * kTeams) + team < items) load(blockIdx.x * kTeams + team, 0);
-    for (int w = blockIdx.x * kTeams + team, n = 0; w < items; w += step, n++) {
+    if (t0 < g.S) load(part == 0);
+    for (int t = t0, n = 0; t < g.S; t += step, n++) {
         parts[team][n & 1][part][lane] = rp.sum();
         team_barrier(team);
-        if (turn == part) {
+        if ((n & 3) == part) {
             if (valid) {
 #pragma unroll
                 for (int d = 0; d < 4; d++) acc -= parts[team][n & 1][d][lane];
@@ -383,8 +437,8 @@ __global__ void __launch_bounds__(kThreads64)
             }
             if (res && p >= 0) res[p + row * np] = (R)acc;
         }
-        turn = (turn + 1) & 3;
-        if (w + step < items) load(w + step, turn);
+        at.next(g);
+        if (t + step < g.S) load(((n + 1) & 3) == part);
     }
     if (NORM) {
 #pragma unroll
@@ -434,22 +488,21 @@ void launch_gs_sweep_dense(const LevelOp<T> &op, const Geom &g, const T *r, T *x
 }
 
 // res = r - A x of a level with per-node rows (res may be null); with partial
-// non-null, per-CTA sums of |r - A x|^2.  Returns the number of CTAs, at most
-// residual_blocks(g).
+// non-null, per-CTA sums of |r - A x|^2.  Returns the number of CTAs: a
+// multiple of 8 (a CTA walks the slots of one colour), two an SM in FP32 and
+// one in FP64 at most.
 template <typename T, typename R>
 int launch_residual_dense(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, R *res, double *partial,
                           cudaStream_t st) {
-    // every CTA walks the slots: two an SM in FP32, one in FP64
+    static_assert(kDensePartials >= 8 * 38);
     if constexpr (sizeof(T) == 4) {
-        int grid = std::min(8 * ((g.S + 31) / 32), 2 * 152);
-        if (partial) grid = std::min(grid, residual_blocks(g));
+        const int grid = 8 * std::min((g.S + 31) / 32, 38);
         if (partial) residual_dense32_kernel<true><<<grid, kThreads32, 0, st>>>(g, op.dop, r, x, res, partial);
         else residual_dense32_kernel<false><<<grid, kThreads32, 0, st>>>(g, op.dop, r, x, res, nullptr);
         return grid;
     } else {
-        const int items = 8 * ((g.S + kNodes64 - 1) / kNodes64);
-        int grid = std::min((items + kTeams - 1) / kTeams, 152);
-        if (partial) grid = std::min(grid, residual_blocks(g));
+        const int items = (g.S + kNodes64 - 1) / kNodes64;
+        const int grid = 8 * std::min((items + kTeams - 1) / kTeams, 19);
         if (partial) residual_dense64_kernel<R, true><<<grid, kThreads64, 0, st>>>(g, op.dop, r, x, res, partial);
         else residual_dense64_kernel<R, false><<<grid, kThreads64, 0, st>>>(g, op.dop, r, x, res, nullptr);
         return grid;

@@ -32,6 +32,7 @@ void launch_gs_sweeps(const LevelOp<T> &op, const Geom &g, const T *r, T *x, T *
 // rows (OP_DENSE); the residual returns its number of norm partials
 template <typename T>
 void launch_gs_sweep_dense(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cudaStream_t st);
+constexpr int kDensePartials = 304;   // at most
 template <typename T, typename R>
 int launch_residual_dense(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, R *res, double *partial,
                           cudaStream_t st);
@@ -116,7 +117,7 @@ void launch_cb_to_nat(const Geom &g, const T *cb, double *nat, cudaStream_t st);
 // natural-order scalar (double) -> colour-blocked scalar
 template <typename T>
 void launch_scalar_nat_to_cb(const Geom &g, const double *nat, T *cb, cudaStream_t st);
-// natural-order dense coefficients (npts x 243 doubles) -> colour-blocked SoA (243 x npad)
+// natural-order dense coefficients (npts x 243 doubles) -> grouped colour-blocked rows (coef_at)
 void launch_coef_nat_to_cb(const Geom &g, const double *nat, double *cb, cudaStream_t st);
 void launch_coef_cb_to_nat(const Geom &g, const double *cb, double *nat, cudaStream_t st);
 void launch_convert(const double *src, float *dst, size_t n, cudaStream_t st);
@@ -179,7 +180,7 @@ template <typename T>
 int tail_cluster_size(int smem_bytes);
 
 // rat.cu
-// Galerkin coarse operator A_c = (1/8) P^T A P into a dense SoA field (243 x npad_c),
+// Galerkin coarse operator A_c = (1/8) P^T A P into grouped rows (coef_at),
 // or, when plane is set, into plane storage (243 x o_c) from the column i = j = 0.
 void launch_rat(const LevelOp<double> &fine, const Geom &gf, const Geom &gc, double *coef_c, bool plane,
                 cudaStream_t st);

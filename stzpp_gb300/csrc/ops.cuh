@@ -190,7 +190,7 @@ constexpr int kPartBlocks = 7;
 template <typename T, bool WITH_CENTRE, bool COH = false>
 __device__ inline void dense_row(const DenseOp<T> &op, const Geom &g, const NbrOffsets &t, int p,
                                  const T *__restrict__ x, T *acc) {
-    const size_t np = (size_t)g.npad;
+    const T *row = op.coef + coef_at(p);
     T part[3] = {T(0), T(0), T(0)};
 #pragma unroll
     for (int b = 0; b < 27; b++) {
@@ -199,9 +199,8 @@ __device__ inline void dense_row(const DenseOp<T> &op, const Geom &g, const NbrO
         if (!(b == 13 && !WITH_CENTRE) && s >= 0) {
             T v[3], a[9];
             load3<T, COH>(x, g.npad, s, v);
-            const T *cb = op.coef + (size_t)(9 * b) * np + p;
 #pragma unroll
-            for (int e = 0; e < 9; e++) a[e] = __ldg(cb + (size_t)e * np);
+            for (int e = 0; e < 9; e++) a[e] = __ldg(row + (9 * b + e) * kCoefGroup);
             if (sizeof(T) == 4) {
                 matvec_sub(a, v, acc);
             } else {

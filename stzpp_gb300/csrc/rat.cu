@@ -75,8 +75,7 @@ __device__ inline void fine_block(const LevelOp<double> &op, const Geom &g, int 
         const int k = fs;   // callers pass the plane index for plane operators
         for (int e = 0; e < 9; e++) a[e] = op.pop.coef[(9 * b + e) * op.pop.O + k];
     } else {
-        const size_t np = (size_t)g.npad;
-        for (int e = 0; e < 9; e++) a[e] = op.dop.coef[(size_t)(9 * b + e) * np + fs];
+        for (int e = 0; e < 9; e++) a[e] = op.dop.coef[coef_at(fs) + (9 * b + e) * kCoefGroup];
     }
 }
 
@@ -148,9 +147,9 @@ __global__ void __launch_bounds__(kRB) rat_kernel(Geom gf, Geom gc, const __grid
             }
         }
     }
-    const size_t np = OUT_PLANE ? (size_t)gc.o : (size_t)gc.npad;
 #pragma unroll
-    for (int e = 0; e < 9; e++) coef_c[(size_t)(9 * off + e) * np + p] = acc[e];
+    for (int e = 0; e < 9; e++)
+        coef_c[OUT_PLANE ? (size_t)(9 * off + e) * gc.o + p : coef_at(p) + (9 * off + e) * kCoefGroup] = acc[e];
 }
 
 template <typename T>
@@ -167,16 +166,15 @@ template <typename T>
 __global__ void dinv_kernel(Geom g, const T *__restrict__ coef, T *__restrict__ dinv, int *bad) {
     int p = blockIdx.x * blockDim.x + threadIdx.x, i, j, k;
     if (p >= g.npad) return;
-    const size_t np = (size_t)g.npad;
-    T a[9], inv[9];
+    T a[9], inv[9], *out = dinv + dinv_at(p);
     if (!slot_node(g, p, i, j, k)) {
-        for (int e = 0; e < 9; e++) dinv[(size_t)e * np + p] = T(0);
+        for (int e = 0; e < 9; e++) out[e * kCoefGroup] = T(0);
         return;
     }
-    for (int e = 0; e < 9; e++) a[e] = coef[(size_t)(9 * 13 + e) * np + p];
+    for (int e = 0; e < 9; e++) a[e] = coef[coef_at(p) + (9 * 13 + e) * kCoefGroup];
     bool ok = inverse3(a, inv);
     if (!ok) atomicExch(bad, 1);
-    for (int e = 0; e < 9; e++) dinv[(size_t)e * np + p] = inv[e];
+    for (int e = 0; e < 9; e++) out[e * kCoefGroup] = inv[e];
 }
 
 // grid_map (region.cc:2587-2604), with the reference's range checks
@@ -275,12 +273,11 @@ __global__ void expand_dense_kernel(Geom g, const __grid_constant__ LevelOp<doub
         }
         fine_block<KIND>(op, g, KIND == OP_PLANE ? k : p, interior, mu_nb, lam_nb, L, b, a);
     }
-    const size_t np = (size_t)g.npad;
-    for (int e = 0; e < 9; e++) coef[(size_t)(9 * b + e) * np + p] = a[e];
+    for (int e = 0; e < 9; e++) coef[coef_at(p) + (9 * b + e) * kCoefGroup] = a[e];
 }
 
 void launch_expand_dense(const LevelOp<double> &op, const Geom &g, double *coef, cudaStream_t st) {
-    cudaMemsetAsync(coef, 0, sizeof(double) * 243 * (size_t)g.npad, st);
+    cudaMemsetAsync(coef, 0, sizeof(double) * coef_len(g.npad), st);
     dim3 grid((g.npad + kRB - 1) / kRB, 27);
     switch (op.kind) {
         case OP_CONST: expand_dense_kernel<OP_CONST><<<grid, kRB, 0, st>>>(g, op, coef); break;
@@ -299,7 +296,7 @@ void launch_rat(const LevelOp<double> &fine, const Geom &gf, const Geom &gc, dou
         else rat_kernel<OP_PLANE, true><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c);
         return;
     }
-    cudaMemsetAsync(coef_c, 0, sizeof(double) * 243 * (size_t)gc.npad, st);
+    cudaMemsetAsync(coef_c, 0, sizeof(double) * coef_len(gc.npad), st);
     dim3 grid((gc.npad + kRB - 1) / kRB, 27);
     switch (fine.kind) {
         case OP_CONST: rat_kernel<OP_CONST, false><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c); break;

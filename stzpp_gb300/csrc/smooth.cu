@@ -81,10 +81,9 @@ __global__ void __launch_bounds__(kBlock) gs_dense_kernel(Geom g, int q, int rev
     load3(r, g.npad, p, acc);
     NbrOffsets nb = nbr_offsets_sub(g, I, J, K, q & 1, (q >> 1) & 1, q >> 2);
     dense_row<T, false>(op, g, nb, p, x, acc);
-    const size_t np = (size_t)g.npad;
     T inv[9];
 #pragma unroll
-    for (int e = 0; e < 9; e++) inv[e] = __ldg(op.dinv + (size_t)e * np + p);
+    for (int e = 0; e < 9; e++) inv[e] = __ldg(op.dinv + dinv_at(p) + e * kCoefGroup);
     x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
     x[p + g.npad] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
     x[p + 2 * g.npad] = dot3(inv[6], acc[0], inv[7], acc[1], inv[8], acc[2]);

@@ -53,7 +53,7 @@ __device__ inline void tail_gs_node(const TailLev<T> &L, int q, int t, const T *
         DenseOp<T> op{L.coef, L.dinv};
         dense_row<T, false, true>(op, g, nb, p, L.x, acc);
 #pragma unroll
-        for (int e = 0; e < 9; e++) inv[e] = __ldg(L.dinv + (size_t)e * g.npad + p);
+        for (int e = 0; e < 9; e++) inv[e] = __ldg(L.dinv + dinv_at(p) + e * kCoefGroup);
     }
     L.x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
     L.x[p + g.npad] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);

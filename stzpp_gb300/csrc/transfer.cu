@@ -187,7 +187,7 @@ __global__ void coef_nat_to_cb_kernel(Geom g, const double *__restrict__ nat, do
     size_t s = slot(g, i, j, k);
     // a Dirichlet node keeps only its centre block (fill_entries stores one entry for it)
     const bool in = is_interior(g, i, j, k);
-    for (int e = 0; e < 243; e++) cb[(size_t)e * g.npad + s] = (in || e / 9 == 13) ? nat[243 * t + e] : 0.0;
+    for (int e = 0; e < 243; e++) cb[coef_at(s) + e * kCoefGroup] = (in || e / 9 == 13) ? nat[243 * t + e] : 0.0;
 }
 
 __global__ void coef_cb_to_nat_kernel(Geom g, const double *__restrict__ cb, double *__restrict__ nat) {
@@ -196,7 +196,7 @@ __global__ void coef_cb_to_nat_kernel(Geom g, const double *__restrict__ cb, dou
     if (t >= npts) return;
     int i = t % g.m, j = (t / g.m) % g.n, k = t / ((long)g.m * g.n);
     size_t s = slot(g, i, j, k);
-    for (int e = 0; e < 243; e++) nat[243 * t + e] = cb[(size_t)e * g.npad + s];
+    for (int e = 0; e < 243; e++) nat[243 * t + e] = cb[coef_at(s) + e * kCoefGroup];
 }
 
 __global__ void convert_kernel(const double *__restrict__ src, float *__restrict__ dst, size_t n) {
