@@ -129,9 +129,19 @@ template <typename T>
 void launch_bottom_direct(int nrow, const double *ainv_t, const int *nat_slot, int npad, const T *r, T *x,
                           cudaStream_t st);
 void launch_scale(double *v, double s, size_t n, cudaStream_t st);
-// inverse of the n x n matrix in the left half of the augmented n x 2n matrix
-// [M | I] (row-major, overwritten) into inv (row-major); bad[0] set when singular
-void launch_gauss_jordan(double *aug, int n, double *inv, int *piv, double *col, int *bad, cudaStream_t st);
+
+// inverse.cu: the n x n matrix of the bottom level in natural node order, 3
+// rows per node, from its grouped rows and box bounds (bad[1] set when a box
+// reaches beyond one node), and its inverse (a is overwritten; both row-major;
+// bad[0] set when singular); pivots: 2 n ints, rows: kInversePanel n doubles of scratch
+constexpr int kInversePanel = 32;
+void launch_bottom_matrix(const Geom &g, const double *coef, const int *S, double *M, int *bad, cudaStream_t st);
+// the same inverse of a plane-invariant bottom level periodic in x and y from
+// its Fourier blocks (scratch: as many doubles as the inverse); false where
+// that does not apply
+bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, double *inv, double *scratch, int *bad,
+                            cudaStream_t st);
+void launch_gauss_jordan(double *a, int n, double *inv, int *pivots, double *rows, int *bad, cudaStream_t st);
 
 // field.cu
 // r (colour-blocked, 3 x npad) = node divergence of the cell tensor field eps

@@ -231,83 +231,6 @@ __global__ void bottom_direct_kernel(int nrow, const double *__restrict__ ainv, 
     if (lane == 0) x[nat_slot[row / 3] + (row % 3) * npad] = (T)acc;
 }
 
-// ---------------------------------------------------------------- bottom inverse
-// Gauss-Jordan elimination with partial pivoting on the augmented matrix
-// [M | I] (n x 2n, row-major, FP64); afterwards the right half is M^-1.
-// Column c: pivot search (one block), row swap + scaling + copy of column c,
-// then elimination of column c from every other row.
-__global__ void gj_pivot_kernel(const double *__restrict__ a, int n, int c, int *piv, int *bad) {
-    __shared__ double bv[1024];
-    __shared__ int bi[1024];
-    double best = -1.0;
-    int arg = c;
-    for (int r = c + threadIdx.x; r < n; r += blockDim.x) {
-        double v = fabs(a[(size_t)r * 2 * n + c]);
-        if (v > best) { best = v; arg = r; }
-    }
-    bv[threadIdx.x] = best;
-    bi[threadIdx.x] = arg;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) {
-            double v2 = bv[threadIdx.x + o];
-            int i2 = bi[threadIdx.x + o];
-            if (v2 > bv[threadIdx.x] || (v2 == bv[threadIdx.x] && i2 < bi[threadIdx.x])) {
-                bv[threadIdx.x] = v2;
-                bi[threadIdx.x] = i2;
-            }
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        *piv = bi[0];
-        if (!(bv[0] > 0.0) || !(bv[0] - bv[0] == 0.0)) atomicExch(bad, 1);
-    }
-}
-
-__global__ void gj_swap_scale_kernel(double *__restrict__ a, int n, int c, const int *piv, double *__restrict__ col) {
-    const int p = *piv;
-    const size_t w = 2 * (size_t)n;
-    // swap rows c and p
-    for (int q = threadIdx.x; q < 2 * n; q += blockDim.x) {
-        double t = a[(size_t)c * w + q];
-        a[(size_t)c * w + q] = a[(size_t)p * w + q];
-        a[(size_t)p * w + q] = t;
-    }
-    __syncthreads();
-    const double inv = 1.0 / a[(size_t)c * w + c];
-    __syncthreads();
-    for (int q = threadIdx.x; q < 2 * n; q += blockDim.x) a[(size_t)c * w + q] *= inv;
-    __syncthreads();
-    for (int r = threadIdx.x; r < n; r += blockDim.x) col[r] = r == c ? 0.0 : a[(size_t)r * w + c];
-}
-
-__global__ void gj_eliminate_kernel(double *__restrict__ a, int n, int c, const double *__restrict__ col) {
-    const size_t w = 2 * (size_t)n;
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = blockIdx.y;
-    if (q >= 2 * n) return;
-    const double f = col[r];
-    if (f != 0.0) a[(size_t)r * w + q] -= f * a[(size_t)c * w + q];
-}
-
-__global__ void gj_extract_kernel(const double *__restrict__ a, int n, double *__restrict__ inv) {
-    size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (t >= (size_t)n * n) return;
-    size_t r = t / n, q = t % n;
-    inv[t] = a[r * 2 * n + n + q];
-}
-
-void launch_gauss_jordan(double *aug, int n, double *inv, int *piv, double *col, int *bad, cudaStream_t st) {
-    dim3 eg((2 * n + 255) / 256, n);
-    for (int c = 0; c < n; c++) {
-        gj_pivot_kernel<<<1, 1024, 0, st>>>(aug, n, c, piv, bad);
-        gj_swap_scale_kernel<<<1, 1024, 0, st>>>(aug, n, c, piv, col);
-        gj_eliminate_kernel<<<eg, 256, 0, st>>>(aug, n, c, col);
-    }
-    gj_extract_kernel<<<(unsigned)(((size_t)n * n + 255) / 256), 256, 0, st>>>(aug, n, inv);
-}
-
 static inline unsigned blocks_for(long n) { return (unsigned)((n + kTB - 1) / kTB); }
 static inline unsigned grid_stride_blocks(size_t n) {
     size_t b = (n + kTB - 1) / kTB;
