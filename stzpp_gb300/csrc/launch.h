@@ -194,6 +194,9 @@ int tail_cluster_size(int smem_bytes);
 // or, when plane is set, into plane storage (243 x o_c) from the column i = j = 0.
 void launch_rat(const LevelOp<double> &fine, const Geom &gf, const Geom &gc, double *coef_c, bool plane,
                 cudaStream_t st);
+// plane storage's largest magnitude outside the structure of coarse_entry, and
+// the largest ratio of it to the plane's largest entry, to out[0], out[1]
+void launch_plane_structure(int O, const double *coef, double *out, cudaStream_t st);
 // inverse centre blocks of plane storage
 template <typename T>
 void launch_plane_dinv(int O, const T *coef, T *dinv, int *bad, cudaStream_t st);

@@ -7,11 +7,15 @@
 //
 // The reference builds A_c = (1/8) P^T A P by scattering, for every fine row
 // f, the row of A P (A_red) into the rows of f's coarse parents.  Here one
-// thread owns one coarse entry (coarse node I, offset J - I) and gathers
+// thread owns coarse entries (coarse node I, offset J - I) and gathers
 //     A_c[I,J] = sum_{f child of I} sum_{g child of J, g in box(f)}
 //                (1/8 A[f,g]) w_P(g,J) w_P(f,I).
 // All weights are powers of two, so every term is bit-identical to the
-// reference's; only the order of the additions differs.  Entries are kept in
+// reference's, and one fused multiply-add by the product of the weights adds
+// it with the rounding of the addition alone; only the order of the additions
+// differs.  (The FP64 pipe bounds the large levels: three products and a sum
+// per term, and a whole Lame row per fine child, took 7.7 ms for the 32x32x33
+// level below a 64x64x65 Lame level; now 1.3 ms.)  Entries are kept in
 // the unwrapped offset convention of the reference's boxes (on a periodic
 // dimension of size 2 or 1, offsets -1 and +1 are separate entries).
 #include "launch.h"
@@ -38,6 +42,9 @@ __device__ inline int wrapd(int a, int len) {
     a %= len;
     return a < 0 ? a + len : a;
 }
+
+// The same for a child of a coarse node: at most one period out.
+__device__ inline int wrap_child(int a, int len) { return a < 0 ? a + len : a >= len ? a - len : a; }
 
 // Block (d) of fine row f for the three operator kinds.
 template <int KIND>
@@ -79,10 +86,31 @@ __device__ inline void fine_block(const LevelOp<double> &op, const Geom &g, int 
     }
 }
 
+// One dimension of a coarse entry: the children f of I, the children g of the
+// target, which of f's neighbours f - 1, f, f + 1 are among them and with
+// what weight (0 for those that are not).
+struct RatDim {
+    int slo, shi, sc, tlo, thi, tc;
+    __device__ __forceinline__ bool set(int I, int off, int mf, int mc, int prd) {
+        children(I, mf, mc, prd, slo, shi, sc);
+        return children(I + off, mf, mc, prd, tlo, thi, tc);
+    }
+    // the weights' exponents: 2^-own, 2^-target, or kNone
+    __device__ __forceinline__ int own(int f) const { return f != sc; }
+    __device__ __forceinline__ int target(int g) const { return g < tlo || g >= thi ? kNone : g != tc; }
+    static constexpr int kNone = 64;
+};
+
+// 2^-n, an integer shift: the FP64 pipe is for the sums.
+__device__ __forceinline__ double weight(int n) { return __longlong_as_double((long long)(1023 - n) << 52); }
+
+// Thread: coarse node p (OUT_PLANE: plane p), offset blockIdx.y, row
+// blockIdx.z of the block.  The nine blocks of one z offset are loaded
+// together: the small levels are bound by the latency of these loads.
 template <int KIND, bool OUT_PLANE>
 __global__ void __launch_bounds__(kRB) rat_kernel(Geom gf, Geom gc, const __grid_constant__ LevelOp<double> op,
                                                   double *__restrict__ coef_c) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x, off = blockIdx.y;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x, off = blockIdx.y, row = blockIdx.z;
     int I, J, K;
     if (OUT_PLANE) {
         // one coarse node per plane: the column i = j = 0
@@ -91,65 +119,181 @@ __global__ void __launch_bounds__(kRB) rat_kernel(Geom gf, Geom gc, const __grid
     } else if (p >= gc.npad || !slot_node(gc, p, I, J, K)) {
         return;
     }
-    const int ox = bdx(off), oy = bdy(off), oz = bdz(off);
-    const int TI = I + ox, TJ = J + oy, TK = K + oz;   // target coarse node (unwrapped)
-    int tlo[3], thi[3], tc[3];
-    if (!children(TI, gf.m, gc.m, gf.xp, tlo[0], thi[0], tc[0]) ||
-        !children(TJ, gf.n, gc.n, gf.yp, tlo[1], thi[1], tc[1]) ||
-        !children(TK, gf.o, gc.o, gf.zp, tlo[2], thi[2], tc[2]))
+    RatDim x, y, z;
+    if (!(x.set(I, bdx(off), gf.m, gc.m, gf.xp) & y.set(J, bdy(off), gf.n, gc.n, gf.yp) &
+          z.set(K, bdz(off), gf.o, gc.o, gf.zp)))
         return;   // entry stays zero
-    int slo[3], shi[3], sc[3];
-    children(I, gf.m, gc.m, gf.xp, slo[0], shi[0], sc[0]);
-    children(J, gf.n, gc.n, gf.yp, slo[1], shi[1], sc[1]);
-    children(K, gf.o, gc.o, gf.zp, slo[2], shi[2], sc[2]);
-    double acc[9];
-#pragma unroll
-    for (int e = 0; e < 9; e++) acc[e] = 0.0;
-    for (int fz = slo[2]; fz < shi[2]; fz++) {
-        const double wfz = fz == sc[2] ? 1.0 : 0.5;
-        const int fzw = wrapd(fz, gf.o);
-        for (int fy = slo[1]; fy < shi[1]; fy++) {
-            const double wfy = fy == sc[1] ? wfz : 0.5 * wfz;
-            const int fyw = wrapd(fy, gf.n);
-            for (int fx = slo[0]; fx < shi[0]; fx++) {
-                const double wf = fx == sc[0] ? wfy : 0.5 * wfy;
-                const int fxw = wrapd(fx, gf.m);
-                const int fs = KIND == OP_PLANE ? fzw : slot(gf, fxw, fyw, fzw);
-                const bool interior = (KIND == OP_DENSE || KIND == OP_PLANE) ? true : is_interior(gf, fxw, fyw, fzw);
-                // box of f: [-1,1]^3 for interior rows (and every dense row), centre only otherwise
-                const int r0 = interior ? -1 : 0, r1 = interior ? 1 : 0;
-                LameRow<double> L;
-                double mu_nb[6], lam_nb[6];
-                if (KIND == OP_LAME && interior) {
-                    NbrOffsets nb = nbr_offsets(gf, fxw, fyw, fzw);
-                    lame_faces(op.lop, gf, nb, fs, L, mu_nb, lam_nb);
+    double acc[3] = {0.0, 0.0, 0.0};
+    for (int fz = z.slo; fz < z.shi; fz++) {
+        const int fzw = wrap_child(fz, gf.o);
+        for (int fy = y.slo; fy < y.shi; fy++) {
+            const int fyw = wrap_child(fy, gf.n);
+            for (int fx = x.slo; fx < x.shi; fx++) {
+                const int wf = 3 + z.own(fz) + y.own(fy) + x.own(fx);   // the 1/8 too
+                const int fxw = wrap_child(fx, gf.m);
+                const double *src;
+                int step = 1;
+                bool interior = true;
+                if (KIND == OP_CONST) {
+                    interior = is_interior(gf, fxw, fyw, fzw);
+                    src = &op.cop.a[0][0];
+                } else if (KIND == OP_PLANE) {
+                    src = op.pop.coef + fzw;
+                    step = op.pop.O;
+                } else {
+                    src = op.dop.coef + coef_at(slot(gf, fxw, fyw, fzw));
+                    step = kCoefGroup;
                 }
-                for (int dz = r0; dz <= r1; dz++) {
-                    const int gz = fz + dz;
-                    if (gz < tlo[2] || gz >= thi[2]) continue;
-                    const double wgz = gz == tc[2] ? 1.0 : 0.5;
-                    for (int dy = r0; dy <= r1; dy++) {
-                        const int gy = fy + dy;
-                        if (gy < tlo[1] || gy >= thi[1]) continue;
-                        const double wgy = gy == tc[1] ? wgz : 0.5 * wgz;
-                        for (int dx = r0; dx <= r1; dx++) {
-                            const int gx = fx + dx;
-                            if (gx < tlo[0] || gx >= thi[0]) continue;
-                            const double wg = gx == tc[0] ? wgy : 0.5 * wgy;
-                            const int b = (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1);
-                            double a[9];
-                            fine_block<KIND>(op, gf, fs, interior, mu_nb, lam_nb, L, b, a);
+                if (!interior) {   // a box of the centre alone
+                    const int n = wf + z.target(fz) + y.target(fy) + x.target(fx);
+                    if (n < RatDim::kNone)
 #pragma unroll
-                            for (int e = 0; e < 9; e++) acc[e] += ((0.125 * a[e]) * wg) * wf;
-                        }
+                        for (int e = 0; e < 3; e++) acc[e] = fma_rn(op.cop.fix[3 * row + e], weight(n), acc[e]);
+                    continue;
+                }
+                for (int dz = max(-1, z.tlo - fz); dz <= min(1, z.thi - 1 - fz); dz++) {
+                    const int wz = wf + z.target(fz + dz);
+                    double a[9][3];
+                    int n[9];
+#pragma unroll
+                    for (int d = 0; d < 9; d++) {
+                        n[d] = wz + y.target(fy + d / 3 - 1) + x.target(fx + d % 3 - 1);
+                        const double *c = src + (size_t)(9 * (9 * (dz + 1) + d) + 3 * row) * step;
+#pragma unroll
+                        for (int e = 0; e < 3; e++) a[d][e] = n[d] < RatDim::kNone ? c[(size_t)e * step] : 0.0;
                     }
+#pragma unroll
+                    for (int d = 0; d < 9; d++)
+                        if (n[d] < RatDim::kNone)
+#pragma unroll
+                            for (int e = 0; e < 3; e++) acc[e] = fma_rn(a[d][e], weight(n[d]), acc[e]);
                 }
             }
         }
     }
 #pragma unroll
-    for (int e = 0; e < 9; e++)
-        coef_c[OUT_PLANE ? (size_t)(9 * off + e) * gc.o + p : coef_at(p) + (9 * off + e) * kCoefGroup] = acc[e];
+    for (int e = 0; e < 3; e++) {
+        const int entry = 9 * off + 3 * row + e;
+        coef_c[OUT_PLANE ? (size_t)entry * gc.o + p : coef_at(p) + entry * kCoefGroup] = acc[e];
+    }
+}
+
+// The same below a Lame level (thread: coarse node p, offset blockIdx.y): of
+// each fine row only the blocks that reach the target, and only their non-zero
+// entries, with lame_faces' and lame_row's arithmetic.
+__global__ void __launch_bounds__(kRB) rat_lame_kernel(Geom gf, Geom gc, LameOp<double> op,
+                                                       double *__restrict__ coef_c) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x, off = blockIdx.y;
+    int I, J, K;
+    if (p >= gc.npad || !slot_node(gc, p, I, J, K)) return;
+    RatDim x, y, z;
+    if (!(x.set(I, bdx(off), gf.m, gc.m, gf.xp) & y.set(J, bdy(off), gf.n, gc.n, gf.yp) &
+          z.set(K, bdz(off), gf.o, gc.o, gf.zp)))
+        return;   // entry stays zero
+    double acc[9];
+#pragma unroll
+    for (int e = 0; e < 9; e++) acc[e] = 0.0;
+    for (int fz = z.slo; fz < z.shi; fz++) {
+        const int fzw = wrap_child(fz, gf.o);
+        for (int fy = y.slo; fy < y.shi; fy++) {
+            const int fyw = wrap_child(fy, gf.n);
+#pragma unroll 1
+            for (int fx = x.slo; fx < x.shi; fx++) {
+                const int wf = 3 + z.own(fz) + y.own(fy) + x.own(fx);   // the 1/8 too
+                const int fxw = wrap_child(fx, gf.m), fs = slot(gf, fxw, fyw, fzw);
+                if (!is_interior(gf, fxw, fyw, fzw)) {   // a box of the centre alone
+                    const int n = wf + z.target(fz) + y.target(fy) + x.target(fx);
+                    if (n < RatDim::kNone) {
+                        const double f = lame_fix(op, fs);
+#pragma unroll
+                        for (int r = 0; r < 3; r++) acc[4 * r] = fma_rn(f, weight(n), acc[4 * r]);
+                    }
+                    continue;
+                }
+                const NbrOffsets t = nbr_offsets_sub(gf, fxw >> 1, fyw >> 1, fzw >> 1, fxw & 1, fyw & 1, fzw & 1);
+                double mu[6], lam[6];
+                const double mu0 = op.mu[fs], lam0 = op.lam[fs];
+#pragma unroll
+                for (int f = 0; f < 6; f++) {
+                    const int s = f & 1 ? 2 : 0, ax = f / 2;
+                    const int nb = t.ox[ax == 0 ? s : 1] + t.oy[ax == 1 ? s : 1] + t.oz[ax == 2 ? s : 1];
+                    mu[f] = op.mu[nb];
+                    lam[f] = op.lam[nb];
+                }
+                int wx[3], wy[3], wz[3];
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    wx[d] = wf + x.target(fx + d - 1);
+                    wy[d] = y.target(fy + d - 1);
+                    wz[d] = z.target(fz + d - 1);
+                }
+                // face f's diagonal entry of component c, without the factor -dt
+                auto face = [&](int f, int c) {
+                    const int ax = f / 2;
+                    const double mu_f = 0.5 * (mu0 + mu[f]), lam_f = 0.5 * (lam0 + lam[f]);
+                    return (c == ax ? (lam_f + 2.0 * mu_f) : mu_f) * op.ih2[ax];
+                };
+#pragma unroll
+                for (int b = 0; b < 27; b++) {
+                    const int dx = bdx(b), dy = bdy(b), dz = bdz(b), nz = nnz_axes(b);
+                    if (nz == 3) continue;
+                    const int n = wx[dx + 1] + wy[dy + 1] + wz[dz + 1];
+                    if (n >= RatDim::kNone) continue;
+                    const double w = weight(n);
+                    if (nz == 0) {
+#pragma unroll
+                        for (int c = 0; c < 3; c++) {
+                            double cen = 0.0;
+#pragma unroll
+                            for (int f = 0; f < 6; f++) cen -= face(f, c);
+                            acc[4 * c] = fma_rn(-op.dt * cen, w, acc[4 * c]);
+                        }
+                    } else if (nz == 1) {
+                        const int f = dx ? (dx > 0 ? 1 : 0) : dy ? (dy > 0 ? 3 : 2) : (dz > 0 ? 5 : 4);
+#pragma unroll
+                        for (int c = 0; c < 3; c++) acc[4 * c] = fma_rn(-op.dt * face(f, c), w, acc[4 * c]);
+                    } else {
+                        const int d[3] = {dx, dy, dz};
+                        const int r = dz == 0 ? 0 : (dy == 0 ? 0 : 1), c = dz == 0 ? 1 : 2;
+                        const double ie = op.iedge[r + c - 1], sgn = d[r] * d[c];
+                        const int nr = 2 * r + (d[r] > 0), nc = 2 * c + (d[c] > 0);
+                        acc[3 * r + c] = fma_rn(-op.dt * ((sgn * (lam[nr] + mu[nc])) * ie), w, acc[3 * r + c]);
+                        acc[3 * c + r] = fma_rn(-op.dt * ((sgn * (lam[nc] + mu[nr])) * ie), w, acc[3 * c + r]);
+                    }
+                }
+            }
+        }
+    }
+    double *out = coef_c + coef_at(p) + 9 * off * kCoefGroup;
+#pragma unroll
+    for (int e = 0; e < 9; e++) out[e * kCoefGroup] = acc[e];
+}
+
+// How far a plane-invariant operator is from the structure of coarse_entry:
+// out[0] the largest magnitude outside it, out[1] the largest ratio of that to
+// a plane's largest entry (both zero before).  A block per 32 planes.
+__global__ void __launch_bounds__(256) plane_structure_kernel(int O, const double *__restrict__ coef, double *out) {
+    __shared__ unsigned long long all[8][32], far[8][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+    unsigned long long a = 0, f = 0;   // bits of magnitudes order as the values
+    if (k < O)
+#pragma unroll 8
+        for (int v = wid; v < 243; v += 8) {
+            const unsigned long long m = __double_as_longlong(coef[(size_t)v * O + k]) & 0x7fffffffffffffffull;
+            a = max(a, m);
+            if (!coarse_entry(v / 9, v % 9)) f = max(f, m);
+        }
+    all[wid][lane] = a;
+    far[wid][lane] = f;
+    __syncthreads();
+    if (wid == 0 && k < O) {
+        for (int w = 1; w < 8; w++) a = max(a, all[w][lane]), f = max(f, far[w][lane]);
+        unsigned long long *o = reinterpret_cast<unsigned long long *>(out);
+        if (f) {
+            atomicMax(o, f);
+            atomicMax(o + 1, (unsigned long long)__double_as_longlong(__longlong_as_double(f) / __longlong_as_double(a)));
+        }
+    }
 }
 
 template <typename T>
@@ -291,19 +435,24 @@ void launch_rat(const LevelOp<double> &fine, const Geom &gf, const Geom &gc, dou
                 cudaStream_t st) {
     if (plane) {
         cudaMemsetAsync(coef_c, 0, sizeof(double) * 243 * (size_t)gc.o, st);
-        dim3 grid((gc.o + kRB - 1) / kRB, 27);
-        if (fine.kind == OP_CONST) rat_kernel<OP_CONST, true><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c);
-        else rat_kernel<OP_PLANE, true><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c);
+        dim3 grid((gc.o + 31) / 32, 27, 3);   // few planes: a warp a block
+        if (fine.kind == OP_CONST) rat_kernel<OP_CONST, true><<<grid, 32, 0, st>>>(gf, gc, fine, coef_c);
+        else rat_kernel<OP_PLANE, true><<<grid, 32, 0, st>>>(gf, gc, fine, coef_c);
         return;
     }
     cudaMemsetAsync(coef_c, 0, sizeof(double) * coef_len(gc.npad), st);
-    dim3 grid((gc.npad + kRB - 1) / kRB, 27);
+    dim3 grid((gc.npad + kRB - 1) / kRB, 27, 3);
     switch (fine.kind) {
         case OP_CONST: rat_kernel<OP_CONST, false><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c); break;
-        case OP_LAME: rat_kernel<OP_LAME, false><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c); break;
+        case OP_LAME: grid.z = 1; rat_lame_kernel<<<grid, kRB, 0, st>>>(gf, gc, fine.lop, coef_c); break;
         case OP_PLANE: rat_kernel<OP_PLANE, false><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c); break;
         default: rat_kernel<OP_DENSE, false><<<grid, kRB, 0, st>>>(gf, gc, fine, coef_c); break;
     }
+}
+
+void launch_plane_structure(int O, const double *coef, double *out, cudaStream_t st) {
+    cudaMemsetAsync(out, 0, 2 * sizeof(double), st);
+    plane_structure_kernel<<<(O + 31) / 32, 256, 0, st>>>(O, coef, out);
 }
 
 template <typename T>
