@@ -92,6 +92,7 @@ struct stz_mg_handle_s {
     int *S[kMaxLev] = {};
     bool bounds_done = false;   // S is filled in
     double *structure = nullptr;   // two numbers per plane-invariant level (launch_plane_structure)
+    int *structured[kMaxLev] = {};   // and a flag per plane
     int top_kind = -1;          // OpKind of the top level once set
     double *mu64 = nullptr, *lam64 = nullptr;
     float *mu32 = nullptr, *lam32 = nullptr;
@@ -598,10 +599,13 @@ void setup(stz_mg_handle h) {
         check_launch();
         h->op64[l] = LevelOp<double>{};
         // the sparsity is known when the levels' structure has been read back below
-        if (plane) launch_plane_structure(gc.o, C.coef, h->structure + 2 * l, h->st);
+        if (plane) {
+            if (!h->structured[l]) h->structured[l] = h->alloc<int>(gc.o);
+            launch_plane_structure(gc.o, C.coef, h->structure + 2 * l, h->structured[l], h->st);
+        }
         if (plane) {
             h->op64[l].kind = OP_PLANE;
-            h->op64[l].pop = PlaneOp<double>{C.coef, C.dinv, gc.o, 0};
+            h->op64[l].pop = PlaneOp<double>{C.coef, C.dinv, gc.o, 0, h->structured[l]};
         } else {
             h->op64[l].kind = OP_DENSE;
             h->op64[l].dop = DenseOp<double>{C.coef, C.dinv};
@@ -621,7 +625,7 @@ void setup(stz_mg_handle h) {
             h->op32[l] = LevelOp<float>{};
             if (plane) {
                 h->op32[l].kind = OP_PLANE;
-                h->op32[l].pop = PlaneOp<float>{F.coef, F.dinv, gc.o, 0};
+                h->op32[l].pop = PlaneOp<float>{F.coef, F.dinv, gc.o, 0, h->structured[l]};
             } else {
                 h->op32[l].kind = OP_DENSE;
                 h->op32[l].dop = DenseOp<float>{F.coef, F.dinv};

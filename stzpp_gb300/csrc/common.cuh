@@ -161,6 +161,8 @@ struct LameOp {
     // expensive, FP64 ones on this GPU especially): 1/h^2 per axis and
     // 1/(4 h_r h_c) per axis pair (x,y), (x,z), (y,z)
     T ih2[3], iedge[3];
+    // the same with their factors: dt/(2 h^2) and dt/(4 h_r h_c)
+    T face[3], edge[3];
 };
 
 template <typename T>
@@ -171,6 +173,10 @@ inline LameOp<T> make_lame_op(const T *mu, const T *lam, double dx, double dy, d
     o.dx = (T)dx; o.dy = (T)dy; o.dz = (T)dz; o.dt = (T)dt;
     o.ih2[0] = (T)(1.0 / (dx * dx)); o.ih2[1] = (T)(1.0 / (dy * dy)); o.ih2[2] = (T)(1.0 / (dz * dz));
     o.iedge[0] = (T)(1.0 / (4.0 * dx * dy)); o.iedge[1] = (T)(1.0 / (4.0 * dx * dz)); o.iedge[2] = (T)(1.0 / (4.0 * dy * dz));
+    for (int a = 0; a < 3; a++) {
+        o.face[a] = (T)(0.5 * dt * (double)o.ih2[a]);
+        o.edge[a] = (T)(dt * (double)o.iedge[a]);
+    }
     return o;
 }
 
@@ -192,12 +198,16 @@ inline size_t dinv_len(size_t npad) { return (npad + kCoefGroup - 1) / kCoefGrou
 // `sparse` marks operators whose entry (r,c) of the block at offset d is zero
 // unless r == c or both d_r and d_c are non-zero (the structure of the
 // Galerkin operators of the constant elasticity stencil: 153 of 243 entries).
+// structured[k]: plane k has that structure, its other entries exactly zero
+// (those of an elasticity stencil between Dirichlet plates do, but for the
+// plates' own planes).
 template <typename T>
 struct PlaneOp {
     const T *coef;
     const T *dinv;
     int O;
     int sparse;
+    const int *structured;
 };
 
 // Round-to-nearest product and fused multiply-add, overloaded on the type.

@@ -36,6 +36,10 @@ constexpr int kDensePartials = 304;   // at most
 template <typename T, typename R>
 int launch_residual_dense(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, R *res, double *partial,
                           cudaStream_t st);
+// plane.cu: one FP64 sweep in place, and the residual, of a plane-invariant level
+void launch_gs_sweep_plane64(const PlaneOp<double> &op, const Geom &g, const double *r, double *x, cudaStream_t st);
+void launch_residual_plane64(const PlaneOp<double> &op, const Geom &g, const double *r, const double *x, double *res,
+                             cudaStream_t st);
 // tile.cu: one sweep reading xin and writing xout (levels periodic in x, y
 // with whole 32x32 tiles, shared-stencil or plane-invariant operators)
 template <typename T>
@@ -195,8 +199,9 @@ int tail_cluster_size(int smem_bytes);
 void launch_rat(const LevelOp<double> &fine, const Geom &gf, const Geom &gc, double *coef_c, bool plane,
                 cudaStream_t st);
 // plane storage's largest magnitude outside the structure of coarse_entry, and
-// the largest ratio of it to the plane's largest entry, to out[0], out[1]
-void launch_plane_structure(int O, const double *coef, double *out, cudaStream_t st);
+// the largest ratio of it to the plane's largest entry, to out[0], out[1];
+// structured[k] = 1 for a plane without any
+void launch_plane_structure(int O, const double *coef, double *out, int *structured, cudaStream_t st);
 // inverse centre blocks of plane storage
 template <typename T>
 void launch_plane_dinv(int O, const T *coef, T *dinv, int *bad, cudaStream_t st);

@@ -271,8 +271,10 @@ __global__ void __launch_bounds__(kRB) rat_lame_kernel(Geom gf, Geom gc, LameOp<
 
 // How far a plane-invariant operator is from the structure of coarse_entry:
 // out[0] the largest magnitude outside it, out[1] the largest ratio of that to
-// a plane's largest entry (both zero before).  A block per 32 planes.
-__global__ void __launch_bounds__(256) plane_structure_kernel(int O, const double *__restrict__ coef, double *out) {
+// a plane's largest entry (both zero before), and the planes with nothing
+// outside it.  A block per 32 planes.
+__global__ void __launch_bounds__(256) plane_structure_kernel(int O, const double *__restrict__ coef, double *out,
+                                                              int *__restrict__ structured) {
     __shared__ unsigned long long all[8][32], far[8][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
     unsigned long long a = 0, f = 0;   // bits of magnitudes order as the values
@@ -289,6 +291,7 @@ __global__ void __launch_bounds__(256) plane_structure_kernel(int O, const doubl
     if (wid == 0 && k < O) {
         for (int w = 1; w < 8; w++) a = max(a, all[w][lane]), f = max(f, far[w][lane]);
         unsigned long long *o = reinterpret_cast<unsigned long long *>(out);
+        structured[k] = f == 0;
         if (f) {
             atomicMax(o, f);
             atomicMax(o + 1, (unsigned long long)__double_as_longlong(__longlong_as_double(f) / __longlong_as_double(a)));
@@ -450,9 +453,9 @@ void launch_rat(const LevelOp<double> &fine, const Geom &gf, const Geom &gc, dou
     }
 }
 
-void launch_plane_structure(int O, const double *coef, double *out, cudaStream_t st) {
+void launch_plane_structure(int O, const double *coef, double *out, int *structured, cudaStream_t st) {
     cudaMemsetAsync(out, 0, 2 * sizeof(double), st);
-    plane_structure_kernel<<<(O + 31) / 32, 256, 0, st>>>(O, coef, out);
+    plane_structure_kernel<<<(O + 31) / 32, 256, 0, st>>>(O, coef, out, structured);
 }
 
 template <typename T>

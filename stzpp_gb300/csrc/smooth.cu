@@ -21,11 +21,15 @@ namespace stzmg {
 
 constexpr int kBlock = 256;
 
-// Colour kernels run on a 3-D grid: block (32, 8), grid (ceil(M2/32),
-// ceil(N2/8), number of sub-grid planes); thread -> sub-grid coordinates
-// (I, J, K) of colour q; the sub-grid planes K in reverse order when rev.
+// Colour kernels run on a 3-D grid, grid z the sub-grid planes K, in reverse
+// order when rev; thread -> sub-grid coordinates (I, J, K) of colour q.  FP32:
+// blocks of 32 x 8, which share more neighbours in L1.  FP64: blocks of 128
+// consecutive slots of the plane, a warp for each of an SM's four schedulers:
+// the FP64 pipe bounds them, where an idle lane at the end of a row costs as
+// much as any (160x96x129, shared stencil, a colour: 31.6 -> %%q%% us).
 #define COLOUR_NODE_PROLOGUE                                                                    \
-    const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y; \
+    int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y;   \
+    if (sizeof(T) == 8) J = I / g.M2, I -= J * g.M2;                                            \
     const int K = rev ? (int)(gridDim.z - 1 - blockIdx.z) : (int)blockIdx.z;                     \
     if (I >= g.M2 || J >= g.N2) return;                                                         \
     const int i = 2 * I + (q & 1), j = 2 * J + ((q >> 1) & 1), k = 2 * K + (q >> 2);             \
@@ -46,6 +50,11 @@ __global__ void __launch_bounds__(kBlock) gs_const_kernel(Geom g, int q, int rev
         inv = op.inv_int;
     } else {
         inv = op.inv_fix;
+    }
+    if (sizeof(T) == 8 && op.centre_diag && inv == op.inv_int) {   // its other entries are zeros
+#pragma unroll
+        for (int e = 0; e < 3; e++) x[p + e * g.npad] = mul_rn(inv[4 * e], acc[e]);
+        return;
     }
     x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
     x[p + g.npad] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
@@ -210,7 +219,7 @@ __device__ inline void block_sum_sq(double v, double *partial) {
         v = tid < kBlock / 32 ? red[tid] : 0.0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (tid == 0) partial[(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = v;
+        if (tid == 0) partial[blockIdx.z * gridDim.x + blockIdx.x] = v;
     }
 }
 
@@ -222,14 +231,16 @@ __global__ void __launch_bounds__(kBlock) residual_kernel(Geom g, const __grid_c
                                                           PlaneOp<T> pop, const T *__restrict__ r,
                                                           const T *__restrict__ x, R *__restrict__ res,
                                                           double *__restrict__ partial) {
-    // block (32, 8): lanes run along x, threadIdx.y is the colour, so a block
-    // covers a 64x2x2 box of nodes in all 8 colours (neighbour reads shared in L1)
+    // block (32, 8): lanes take 32 consecutive slots of a sub-grid plane (across
+    // the ends of rows: an idle lane costs the FP64 pipe as much as a busy one),
+    // threadIdx.y is the colour, so a block covers the 8 colours of 32 2x2x2
+    // boxes of nodes (neighbour reads shared in L1)
     const int q = threadIdx.y;
-    const int I = blockIdx.x * 32 + threadIdx.x, J = blockIdx.y, K = blockIdx.z;
+    const int t = blockIdx.x * 32 + threadIdx.x, J = t / g.M2, I = t - J * g.M2, K = blockIdx.z;
     const int a = q & 1, b = (q >> 1) & 1, c = q >> 2;
     const int i = 2 * I + a, j = 2 * J + b, k = 2 * K + c;
     double sq = 0.0;
-    if (I < g.M2) {
+    if (J < g.N2) {
         const int p = q * g.S + (K * g.N2 + J) * g.M2 + I;
         T acc[3] = {T(0), T(0), T(0)};
         if (i < g.m && j < g.n && k < g.o) {
@@ -289,7 +300,9 @@ void launch_sum_partials(const double *partial, int n, double *out, cudaStream_t
 template <typename T>
 static void launch_gs_colour_planes(const LevelOp<T> &op, const Geom &g, int q, int rev, const T *r, T *x,
                                     cudaStream_t st) {
-    const dim3 blocks((g.M2 + 31) / 32, (g.N2 + 7) / 8, g.O2), blk(32, 8);
+    const bool flat = sizeof(T) == 8;
+    const dim3 blk = flat ? dim3(128) : dim3(32, 8);
+    const dim3 blocks = flat ? dim3((g.M2 * g.N2 + 127) / 128, 1, g.O2) : dim3((g.M2 + 31) / 32, (g.N2 + 7) / 8, g.O2);
     switch (op.kind) {
         case OP_CONST:
             if (op.cop.elastic) gs_const_kernel<T, true><<<blocks, blk, 0, st>>>(g, q, rev, op.cop, r, x);
@@ -321,7 +334,8 @@ static bool odd_periodic_z(const Geom &g) { return g.zp && (g.o & 1) && g.o > 1;
 
 template <typename T>
 static bool large_planes(const LevelOp<T> &op, const Geom &g) {
-    if (op.kind == OP_DENSE) return odd_periodic_z(g);   // dense.cu takes planes of any size
+    // dense.cu and plane.cu take planes of any size
+    if (op.kind == OP_DENSE || (op.kind == OP_PLANE && sizeof(T) == 8)) return odd_periodic_z(g);
     const int phase_max = sizeof(T) == 8 ? 256 : 2 * kPhaseThreads;   // FP64 needs every SM's FP64 units
     return odd_periodic_z(g) || g.M2 * g.N2 > phase_max;
 }
@@ -371,7 +385,8 @@ void launch_gs_sweep(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cuda
             break;
         case OP_LAME: launch_phases<T, OP_LAME, false, false>(op, g, r, x, st); break;
         case OP_PLANE:
-            if (op.pop.sparse) launch_phases<T, OP_PLANE, false, true>(op, g, r, x, st);
+            if constexpr (sizeof(T) == 8) launch_gs_sweep_plane64(op.pop, g, r, x, st);
+            else if (op.pop.sparse) launch_phases<T, OP_PLANE, false, true>(op, g, r, x, st);
             else launch_phases<T, OP_PLANE, false, false>(op, g, r, x, st);
             break;
         default: launch_gs_sweep_dense<T>(op, g, r, x, st); break;
@@ -383,7 +398,7 @@ int residual_blocks(const Geom &g) { return ((g.M2 + 31) / 32) * g.N2 * g.O2; }
 template <typename T, typename R, bool NORM>
 static void launch_residual_k(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, R *res, double *partial,
                               cudaStream_t st) {
-    const dim3 blocks((g.M2 + 31) / 32, g.N2, g.O2), blk(32, 8);
+    const dim3 blocks((g.M2 * g.N2 + 31) / 32, 1, g.O2), blk(32, 8);
     switch (op.kind) {
         case OP_CONST:
             if (op.cop.elastic)
@@ -418,9 +433,15 @@ void launch_residual(const LevelOp<T> &op, const Geom &g, const T *r, const T *x
         if (partial && out) sum_partials_kernel<<<1, 1024, 0, st>>>(partial, nb, out);
         return;
     }
+    if constexpr (std::is_same<R, double>::value) {
+        if (op.kind == OP_PLANE && res && !partial) {
+            launch_residual_plane64(op.pop, g, r, x, res, st);
+            return;
+        }
+    }
     if (partial) launch_residual_k<T, R, true>(op, g, r, x, res, partial, st);
     else launch_residual_k<T, R, false>(op, g, r, x, res, partial, st);
-    if (partial && out) sum_partials_kernel<<<1, 1024, 0, st>>>(partial, residual_blocks(g), out);
+    if (partial && out) sum_partials_kernel<<<1, 1024, 0, st>>>(partial, (g.M2 * g.N2 + 31) / 32 * g.O2, out);
 }
 
 template void launch_gs_colour<float>(const LevelOp<float> &, const Geom &, int, const float *, float *, cudaStream_t);
