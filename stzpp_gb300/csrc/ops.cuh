@@ -121,10 +121,70 @@ __device__ inline void lame_faces(const LameOp<T> &op, const Geom &g, const NbrO
     for (int c = 0; c < 3; c++) L.centre[c] = -op.dt * cen[c];
 }
 
+// The same row in FP64, whose pipe bounds it: the factors dt/h^2 enter once
+// per axis and pair instead of once per entry, 117 instructions for 187.
+template <bool WITH_CENTRE>
+__device__ inline void lame_row64(const LameOp<double> &op, const Geom &g, const NbrOffsets &t, int p,
+                                  const double *__restrict__ x, double *acc, double *centre_out) {
+    const int npad = g.npad;
+    const int mid = t.ox[1] + t.oy[1] + t.oz[1];
+    const double mu0 = op.mu[p], lam0 = op.lam[p];
+    double mu[6], lam[6], cen[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int ax = 0; ax < 3; ax++) {
+        double s[2], w[2], v[2][3];   // mu0 + mu, lam0 + lam + 2 (mu0 + mu) and x of the faces below and above
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int *o = ax == 0 ? t.ox : ax == 1 ? t.oy : t.oz;
+            const int sl = mid - o[1] + o[2 * u];
+            mu[2 * ax + u] = op.mu[sl];
+            lam[2 * ax + u] = op.lam[sl];
+            load3(x, npad, sl, v[u]);
+            s[u] = mu0 + mu[2 * ax + u];
+            w[u] = fma_rn(2.0, s[u], lam0 + lam[2 * ax + u]);
+        }
+        const double ss = s[0] + s[1], ws = w[0] + w[1];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const double lo = c == ax ? w[0] : s[0], hi = c == ax ? w[1] : s[1];
+            acc[c] = fma_rn(op.face[ax], fma_rn(hi, v[1][c], mul_rn(lo, v[0][c])), acc[c]);
+            cen[c] = fma_rn(op.face[ax], c == ax ? ws : ss, cen[c]);
+        }
+    }
+#pragma unroll
+    for (int pr = 0; pr < 3; pr++) {
+        const int r = pr == 2 ? 1 : 0, c = pr == 0 ? 1 : 2;
+        double er = 0.0, ec = 0.0;
+#pragma unroll
+        for (int ir = 0; ir < 2; ir++)
+#pragma unroll
+            for (int ic = 0; ic < 2; ic++) {
+                int d[3] = {1, 1, 1};
+                d[r] = 2 * ir;
+                d[c] = 2 * ic;
+                const int sl = t.ox[d[0]] + t.oy[d[1]] + t.oz[d[2]];
+                const double a = lam[2 * r + ir] + mu[2 * c + ic], b = lam[2 * c + ic] + mu[2 * r + ir];
+                er = fma_rn(ir == ic ? a : -a, x[sl + c * npad], er);
+                ec = fma_rn(ir == ic ? b : -b, x[sl + r * npad], ec);
+            }
+        acc[r] = fma_rn(op.edge[pr], er, acc[r]);
+        acc[c] = fma_rn(op.edge[pr], ec, acc[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        if (WITH_CENTRE) acc[c] = fma_rn(-cen[c], x[p + c * npad], acc[c]);
+        if (centre_out) centre_out[c] = cen[c];
+    }
+}
+
 // acc -= sum over the 18 non-zero off-centre blocks (and the centre if asked).
 template <typename T, bool WITH_CENTRE>
 __device__ inline void lame_row(const LameOp<T> &op, const Geom &g, const NbrOffsets &t, int p,
                                 const T *__restrict__ x, T *acc, T *centre_out) {
+    if constexpr (sizeof(T) == 8) {
+        lame_row64<WITH_CENTRE>(op, g, t, p, x, acc, centre_out);
+        return;
+    }
     LameRow<T> L;
     T mu_nb[6], lam_nb[6];
     lame_faces(op, g, t, p, L, mu_nb, lam_nb);

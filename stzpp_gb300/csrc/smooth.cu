@@ -26,7 +26,7 @@ constexpr int kBlock = 256;
 // blocks of 32 x 8, which share more neighbours in L1.  FP64: blocks of 128
 // consecutive slots of the plane, a warp for each of an SM's four schedulers:
 // the FP64 pipe bounds them, where an idle lane at the end of a row costs as
-// much as any (160x96x129, shared stencil, a colour: 31.6 -> %%q%% us).
+// much as any (160x96x129, shared stencil, a colour: 31.6 -> 25.2 us).
 #define COLOUR_NODE_PROLOGUE                                                                    \
     int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y;   \
     if (sizeof(T) == 8) J = I / g.M2, I -= J * g.M2;                                            \
