@@ -214,18 +214,36 @@ __global__ void scale_kernel(double *__restrict__ v, double s, size_t n) {
     for (; t < n; t += (size_t)gridDim.x * blockDim.x) v[t] *= s;
 }
 
-// x = Ainv r with one warp per row (Ainv row-major, lanes stride the columns).
+// FP32 to FP64 by the bits where the value is a normal number: a conversion
+// takes the FP64 pipe as long as a product.
+__device__ __forceinline__ double widen(float v) {
+    const unsigned u = __float_as_uint(v), e = u >> 23 & 255;
+    if (e - 1 > 253) return (double)v;
+    return __hiloint2double((int)((u & 0x80000000u) | ((u & 0x7fffffffu) >> 3) + 0x38000000u), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
+// x = Ainv r, a warp per row (Ainv row-major, lanes stride the columns), a row
+// per scheduler and block.  r is gathered and widened once per block: a look-up
+// and an FP64 conversion per matrix entry took the 1728-row product of an FP32
+// cycle 17.6 us with the matrix in L2, 25.7 us without, the FP64 pipe's share
+// of the products being 5; now 10.9 and 15.9 us.
+constexpr int kBottomRows = 4;
+
 template <typename T>
-__global__ void bottom_direct_kernel(int nrow, const double *__restrict__ ainv, const int *__restrict__ nat_slot,
-                                     int npad, const T *__restrict__ r, T *__restrict__ x) {
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(32 * kBottomRows)
+    bottom_direct_kernel(int nrow, const double *__restrict__ ainv, const int *__restrict__ nat_slot, int npad,
+                         const T *__restrict__ r, T *__restrict__ x) {
+    extern __shared__ double rn[];
+    const int lane = threadIdx.x & 31, row = blockIdx.x * kBottomRows + (threadIdx.x >> 5);
+#pragma unroll 4
+    for (int col = threadIdx.x; col < nrow; col += 32 * kBottomRows) rn[col] = widen(r[nat_slot[col / 3] + (col % 3) * npad]);
+    __syncthreads();
     if (row >= nrow) return;
     double acc = 0.0;
     const double *a = ainv + (size_t)row * nrow;
-    for (int col = lane; col < nrow; col += 32) {
-        int s = nat_slot[col / 3] + (col % 3) * npad;
-        acc += a[col] * (double)r[s];
-    }
+#pragma unroll 16
+    for (int col = lane; col < nrow; col += 32) acc += a[col] * rn[col];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if (lane == 0) x[nat_slot[row / 3] + (row % 3) * npad] = (T)acc;
@@ -277,7 +295,11 @@ void launch_scale(double *v, double s, size_t n, cudaStream_t st) {
 template <typename T>
 void launch_bottom_direct(int nrow, const double *ainv_t, const int *nat_slot, int npad, const T *r, T *x,
                           cudaStream_t st) {
-    bottom_direct_kernel<T><<<blocks_for(32L * nrow), kTB, 0, st>>>(nrow, ainv_t, nat_slot, npad, r, x);
+    const int smem = nrow * (int)sizeof(double);   // 96 KB at the 4096 nodes a direct bottom may have
+    if (smem > 48 * 1024)
+        cudaFuncSetAttribute(bottom_direct_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    bottom_direct_kernel<T><<<(nrow + kBottomRows - 1) / kBottomRows, 32 * kBottomRows, smem, st>>>(nrow, ainv_t, nat_slot,
+                                                                                                  npad, r, x);
 }
 
 template void launch_restriction<float>(const Geom &, const Geom &, const float *, float *, cudaStream_t);
