@@ -312,6 +312,10 @@ void set_const_op(stz_mg_handle h, const double *stencil, const double *fix) {
         for (int e = 0; e < 9; e++)
             if (!elastic_entry(b, e) && c.a[b][e] != 0.0) elastic = 0;
     c.elastic = elastic;
+    c.corners = 0;
+    for (int b = 0; b < 27; b++)
+        for (int e = 0; e < 9; e++)
+            if (nnz_axes(b) == 3 && c.a[b][e] != 0.0) c.corners = 1;
     c.centre_diag = c.a[13][1] == 0.0 && c.a[13][2] == 0.0 && c.a[13][3] == 0.0 && c.a[13][5] == 0.0 &&
                     c.a[13][6] == 0.0 && c.a[13][7] == 0.0;
     ConstOp<float> f{};
@@ -323,6 +327,7 @@ void set_const_op(stz_mg_handle h, const double *stencil, const double *fix) {
         f.inv_fix[e] = (float)c.inv_fix[e];
     }
     f.elastic = elastic;
+    f.corners = c.corners;
     f.centre_diag = c.centre_diag;
     h->op64[0] = LevelOp<double>{};
     h->op64[0].kind = OP_CONST;

@@ -60,6 +60,12 @@ constexpr int kOwnSub = band_rows(M2) / 2;      // sub-grid rows per parity owne
 template <int M2>
 constexpr int kStageRows = kOwnSub<M2> + 2;     // staged sub-rows J0-1 .. J0+kOwnSub
 
+// Sub-grid columns of a level: M2, or fewer where its rows are staged padded to M2.
+template <int M2, bool PAD>
+__device__ __forceinline__ int band_width(const Geom &g) {
+    return PAD ? g.M2 : M2;
+}
+
 // Shared-memory layout of the staged band: plane p (0: k-1, 1: k, 2: k+1),
 // component c, sub-row Jr (staged row 0 is sub-row J0-1), colour ab = a + 2b
 // of the plane, sub-grid column I: Jr outside ab, so one TMA box brings a
@@ -206,11 +212,12 @@ __device__ __forceinline__ void stage_coef(const PlaneOp<T> &pop, int k, T *cfs,
 // at column I + floor((A+dx)/2) (wrapped: base index ib[0..2] for shifts -1,
 // 0, +1, which already include the rows T0) and staged row
 // Jr + floor((B+dy)/2), Jr = t + 1.
-// KIND: OP_CONST (the elasticity stencil shared by every interior node, op.cop)
-// or OP_PLANE (the row of coefficients of plane k, cf: 243 entries and the 9
-// of the inverse centre block, in shared memory; SPARSE: the structural
-// zeros of the coarse elasticity operators), with the arithmetic of
-// const_row<T, true, false> or plane_row_coef<T, SPARSE, false>.
+// KIND: OP_CONST (the stencil shared by every interior node, op.cop; SPARSE:
+// the elasticity stencil, else full blocks) or OP_PLANE (the row of
+// coefficients of plane k, cf: 243 entries and the 9 of the inverse centre
+// block, in shared memory; SPARSE: the structural zeros of the coarse
+// elasticity operators), with the arithmetic of const_row<T, SPARSE, false> or
+// plane_row_coef<T, SPARSE, false>.
 template <typename T, int M2, int KIND, bool SPARSE, int A, int B, int NR>
 __device__ __forceinline__ void band_colour(const T *__restrict__ s, const int (&ib)[3], const LevelOp<T> &op,
                                             const T *cf, int nvalid, const T (&rr)[NR][3], T (&out)[NR][3]) {
@@ -289,8 +296,30 @@ __device__ __forceinline__ void band_colour(const T *__restrict__ s, const int (
     }
 #pragma unroll
     for (int u = 0; u < NR; u++) {
-        if (u >= nvalid) break;   // warp-uniform
+        if (u >= nvalid) break;
         const int Jr = u + 1;
+        if constexpr (!SPARSE) {   // full blocks: three values and matvec_sub at a time
+            T acc[3] = {rr[u][0], rr[u][1], rr[u][2]};
+            sfor<0, 27>([&](auto bi) {
+                constexpr int b = decltype(bi)::value;
+                if constexpr (b != 13) {
+                    constexpr int dx = bdx(b), dy = bdy(b), dz = bdz(b);
+                    constexpr int ap = (A + dx + 2) & 1, sI = (A + dx + 2) / 2 - 1;
+                    constexpr int bp = (B + dy + 2) & 1, sJ = (B + dy + 2) / 2 - 1;
+                    if (nnz_axes(b) == 3 && !op.cop.corners) return;   // products of zeros
+                    T v[3];
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+                        v[c] = s[ib[sI + 1] + woff<M2>(1 + dz, c, 0, ap + 2 * bp, 0) + (Jr + sJ) * rowstep];
+                    matvec_sub(op.cop.a[b], v, acc);
+                }
+            });
+            const T *inv = op.cop.inv_int;
+            out[u][0] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
+            out[u][1] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
+            out[u][2] = dot3(inv[6], acc[0], inv[7], acc[1], inv[8], acc[2]);
+            continue;
+        }
         T v[27][3];
         sfor<0, 27>([&](auto bi) {
             constexpr int b = decltype(bi)::value;
@@ -379,10 +408,11 @@ __device__ __forceinline__ void band_issue(const BandArgs &args, const BandMaps 
 }
 
 // A Dirichlet plate of the shared stencil: x = fix^-1 r, no neighbours.
-template <typename T, int M2, int NH>
+template <typename T, int M2, int NH, bool PAD>
 __device__ __forceinline__ void band_plate(const Geom &g, const ConstOp<T> &op, const BandItem &it, int c,
                                            const T *__restrict__ r, T *__restrict__ xout) {
     const int tid = threadIdx.x, I = tid % M2, hh = tid / M2;
+    if (PAD && I >= g.M2) return;
     const size_t np = (size_t)g.npad;
     const T *inv = op.inv_fix;
 #pragma unroll 1
@@ -400,7 +430,7 @@ __device__ __forceinline__ void band_plate(const Geom &g, const ConstOp<T> &op, 
 // boxes are in flight), the wait for the boxes (phase `phase` of bar, at
 // most 0.2 s), then the plane's four colours.  False if the boxes did not
 // arrive (recorded; every thread returns false).
-template <typename T, int M2, int NH, int KIND, bool SPARSE>
+template <typename T, int M2, int NH, int KIND, bool SPARSE, bool PAD>
 __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp<T> &op, const BandItem &it, T *s,
                                              T *cfs, unsigned bar, unsigned phase, const T *__restrict__ r,
                                              T *__restrict__ xout) {
@@ -412,7 +442,8 @@ __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp
     constexpr int OWN = kOwnSub<M2>;
     constexpr int P0 = kPer<OWN + 1, NH>, P1 = kPer<OWN, NH>;
     const int t0a = hh * P0, t0b = hh * P1;
-    const int na = min(P0, OWN + 1 - t0a), nb = min(P1, OWN - t0b);
+    const bool column = !PAD || I < g.M2;   // the padding's columns have no rows
+    const int na = column ? min(P0, OWN + 1 - t0a) : 0, nb = column ? min(P1, OWN - t0b) : 0;
     T r0[P0][3], r1[P0][3], r2[P1][3], r3[P1][3];
 #pragma unroll
     for (int u = 0; u < P0; u++) {
@@ -456,7 +487,8 @@ __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp
         __syncthreads();
     }
     constexpr int rowstep = woff<M2>(0, 0, 1, 0, 0);
-    const int ibx[3] = {I == 0 ? M2 - 1 : I - 1, I, I == M2 - 1 ? 0 : I + 1};
+    const int width = band_width<M2, PAD>(g);
+    const int ibx[3] = {I == 0 ? width - 1 : I - 1, I, I == width - 1 ? 0 : I + 1};
     const int iba[3] = {ibx[0] + t0a * rowstep, ibx[1] + t0a * rowstep, ibx[2] + t0a * rowstep};
     const int ibb[3] = {ibx[0] + t0b * rowstep, ibx[1] + t0b * rowstep, ibx[2] + t0b * rowstep};
     // store a colour's new values: shared memory for the later colours, x_out
@@ -513,9 +545,9 @@ __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp
 // 8-row bands); one elsewhere (ptxas then keeps every value in registers).
 template <typename T, int M2, int KIND>
 constexpr int kBandMinBlocks =
-    sizeof(T) == 4 && M2 >= 128 ? (KIND == OP_CONST ? 233472 / (kBandWords<M2> * 4 + 2048) : 2) : 1;
+    sizeof(T) == 4 && M2 >= 96 ? (KIND == OP_CONST ? 233472 / (kBandWords<M2> * 4 + 2048) : 2) : 1;
 
-template <typename T, int M2, int NH, int KIND, bool SPARSE>
+template <typename T, int M2, int NH, int KIND, bool SPARSE, bool PAD>
 __global__ void __launch_bounds__(NH * M2, (kBandMinBlocks<T, M2, KIND>))
     gs_band_kernel(const BandArgs args, const __grid_constant__ LevelOp<T> op, const __grid_constant__ BandMaps in,
                    const __grid_constant__ BandMaps out_maps, const T *__restrict__ r, T *__restrict__ xout) {
@@ -525,7 +557,7 @@ __global__ void __launch_bounds__(NH * M2, (kBandMinBlocks<T, M2, KIND>))
     const int tid = threadIdx.x;
     const BandItem it = band_item<M2>(args, blockIdx.x);
     if (!band_stages<KIND>(it)) {
-        band_plate<T, M2, NH>(args.g, op.cop, it, args.c, r, xout);
+        band_plate<T, M2, NH, PAD>(args.g, op.cop, it, args.c, r, xout);
         return;
     }
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(band_smem);
@@ -540,7 +572,7 @@ __global__ void __launch_bounds__(NH * M2, (kBandMinBlocks<T, M2, KIND>))
     }
     __syncthreads();
     if (tid == 0) band_issue<T, M2>(args, in, out_maps, it, sbase, bar);
-    band_compute<T, M2, NH, KIND, SPARSE>(args, op, it, reinterpret_cast<T *>(band_smem), cfs, bar, 0, r, xout);
+    band_compute<T, M2, NH, KIND, SPARSE, PAD>(args, op, it, reinterpret_cast<T *>(band_smem), cfs, bar, 0, r, xout);
 }
 
 // ------------------------------------------------------------ residual
@@ -662,8 +694,8 @@ __device__ __forceinline__ void band_res_colour(const T *__restrict__ s, const i
     }
 }
 
-template <typename T, int M2, int NH, int KIND, bool SPARSE>
-__global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 128 ? 2 : 1)
+template <typename T, int M2, int NH, int KIND, bool SPARSE, bool PAD>
+__global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 96 ? 2 : 1)
     residual_band_kernel(const BandArgs args, const __grid_constant__ LevelOp<T> op,
                          const __grid_constant__ BandMaps xm, const T *__restrict__ r, T *__restrict__ res) {
     extern __shared__ __align__(128) unsigned char band_smem[];
@@ -677,7 +709,7 @@ __global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 128 ? 2 : 1)
     const bool has_lo = g.zp || k > 0, has_hi = g.zp || k < g.o - 1;
     if (KIND == OP_CONST && !(has_lo && has_hi)) {   // a Dirichlet plate: r - fix x
 #pragma unroll 1
-        for (int w = hh; w < 4 * kOwnSub<M2>; w += NH) {
+        for (int w = hh; w < 4 * kOwnSub<M2> && (!PAD || I < g.M2); w += NH) {
             const int ab = w / kOwnSub<M2>, t = w % kOwnSub<M2>;
             const size_t sl = band_slot(g, ab, c, K, J0 + t, I);
             T acc[3] = {r[sl], r[sl + np], r[sl + 2 * np]};
@@ -729,8 +761,9 @@ __global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 128 ? 2 : 1)
         __syncthreads();
     }
     constexpr int P = kPer<kOwnSub<M2>, NH>;
-    const int t0 = hh * P, nv = min(P, kOwnSub<M2> - t0);
-    const int ib[3] = {I == 0 ? M2 - 1 : I - 1, I, I == M2 - 1 ? 0 : I + 1};
+    const int t0 = hh * P, nv = !PAD || I < g.M2 ? min(P, kOwnSub<M2> - t0) : 0;
+    const int width = band_width<M2, PAD>(g);
+    const int ib[3] = {I == 0 ? width - 1 : I - 1, I, I == width - 1 ? 0 : I + 1};
     // the four colours as the branches of a loop that is not unrolled: the
     // colours share no barrier, and in one straight run the instruction
     // scheduler would start every colour's shared loads at once
@@ -769,11 +802,11 @@ EncodeTiled encoder() {
 
 // The tensor maps of one colour-blocked field of level g: a 5-d view with
 // column I innermost, then colour ab, sub-row J, plane K, component x plane
-// parity, and boxes of the whole row of M2 columns, 4 colours and 6, 5 or 1
-// sub-rows.  False if the driver does not accept them (the caller then runs
-// the colour launches).
+// parity, and boxes of a row padded to `pad` columns (those beyond the grid
+// arrive as zeros), 4 colours and 6, 5 or 1 sub-rows.  False if the driver
+// does not accept them (the caller then runs the colour launches).
 template <typename T>
-bool make_band_maps(const Geom &g, const T *field, BandMaps &mp) {
+bool make_band_maps(const Geom &g, int pad, const T *field, BandMaps &mp) {
     EncodeTiled enc = encoder();
     if (!enc) return false;
     const cuuint64_t e = sizeof(T);
@@ -785,7 +818,7 @@ bool make_band_maps(const Geom &g, const T *field, BandMaps &mp) {
     const cuuint32_t stage = (cuuint32_t)(band_rows(g.M2) / 2 + 2);
     const cuuint32_t rows[3] = {stage, stage - 1, 1};
     for (int i = 0; i < 3; i++) {
-        const cuuint32_t box[5] = {(cuuint32_t)M2, 4, rows[i], 1, 1};
+        const cuuint32_t box[5] = {(cuuint32_t)pad, 4, rows[i], 1, 1};
         if (enc(maps[i], dt, 5, const_cast<T *>(field), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -809,11 +842,11 @@ bool first_band_use(unsigned long long &devices) {
 template <typename T, int M2>
 constexpr int kResNH = 2;
 
-template <typename T, int M2, int NH, int KIND, bool SPARSE>
+template <typename T, int M2, int NH, int KIND, bool SPARSE, bool PAD>
 bool launch_band_kn(const LevelOp<T> &op, const Geom &g, const T *r, const T *xin, T *xout, cudaStream_t st) {
     BandMaps min_, mout;
-    if (!make_band_maps<T>(g, xin, min_) || !make_band_maps<T>(g, xout, mout)) return false;
-    auto kern = gs_band_kernel<T, M2, NH, KIND, SPARSE>;
+    if (!make_band_maps<T>(g, M2, xin, min_) || !make_band_maps<T>(g, M2, xout, mout)) return false;
+    auto kern = gs_band_kernel<T, M2, NH, KIND, SPARSE, PAD>;
     const int smem = kBandWords<M2> * (int)sizeof(T);
     static unsigned long long attr_devices = 0;
     if (first_band_use(attr_devices)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -843,26 +876,47 @@ bool launch_band_kn(const LevelOp<T> &op, const Geom &g, const T *r, const T *xi
 // latency of each thread's chain (mixed solve 21.99 -> 21.65 ms against four
 // on the 16- and 8-column levels, 21.73 -> 21.68 ms on the 32-column one);
 // one or two in FP64 (registers).
-template <typename T, int M2, int KIND, bool SPARSE>
+template <typename T, int M2, int KIND, bool SPARSE, bool PAD = false>
 bool launch_band_k(const LevelOp<T> &op, const Geom &g, const T *r, const T *xin, T *xout, cudaStream_t st) {
     constexpr int NH = sizeof(T) == 4 ? (M2 >= 64 ? 2 : 8) : (M2 >= 64 ? 1 : 2);
-    return launch_band_kn<T, M2, NH, KIND, SPARSE>(op, g, r, xin, xout, st);
+    return launch_band_kn<T, M2, NH, KIND, SPARSE, PAD>(op, g, r, xin, xout, st);
+}
+
+// The width a level's rows are staged with (0: too wide): their own where a
+// kernel is compiled for it (the width at run time costs the 128-column sweep
+// 2 %), else the next of those that allow for padding, FP32 only.
+template <typename T>
+int band_pad(int M2) {
+    for (int p : {8, 16, 32, 64, 128})
+        if (M2 == p) return p;
+    for (int p : {24, 48, 96, 128})
+        if (sizeof(T) == 4 && M2 >= 8 && M2 <= p) return p;
+    return 0;
 }
 
 template <typename T, int KIND, bool SPARSE>
 bool launch_band_m(const LevelOp<T> &op, const Geom &g, const T *r, const T *xin, T *xout, cudaStream_t st) {
-    switch (g.M2) {
+    switch (band_pad<T>(g.M2)) {
         case 8: return launch_band_k<T, 8, KIND, SPARSE>(op, g, r, xin, xout, st);
         case 16: return launch_band_k<T, 16, KIND, SPARSE>(op, g, r, xin, xout, st);
         case 32: return launch_band_k<T, 32, KIND, SPARSE>(op, g, r, xin, xout, st);
         case 64: return launch_band_k<T, 64, KIND, SPARSE>(op, g, r, xin, xout, st);
-        case 128: return launch_band_k<T, 128, KIND, SPARSE>(op, g, r, xin, xout, st);
-        default: return false;
+        case 128: if (g.M2 == 128) return launch_band_k<T, 128, KIND, SPARSE>(op, g, r, xin, xout, st);
     }
+    if constexpr (sizeof(T) == 4) {
+        switch (band_pad<T>(g.M2)) {
+            case 24: return launch_band_k<T, 24, KIND, SPARSE, true>(op, g, r, xin, xout, st);
+            case 48: return launch_band_k<T, 48, KIND, SPARSE, true>(op, g, r, xin, xout, st);
+            case 96: return launch_band_k<T, 96, KIND, SPARSE, true>(op, g, r, xin, xout, st);
+            case 128: return launch_band_k<T, 128, KIND, SPARSE, true>(op, g, r, xin, xout, st);
+        }
+    }
+    return false;
 }
 
 template <typename T>
 bool launch_band_op(const LevelOp<T> &op, const Geom &g, const T *r, const T *xin, T *xout, cudaStream_t st) {
+    if (op.kind == OP_CONST && op.cop.elastic) return launch_band_m<T, OP_CONST, true>(op, g, r, xin, xout, st);
     if (op.kind == OP_CONST) return launch_band_m<T, OP_CONST, false>(op, g, r, xin, xout, st);
     if (op.pop.sparse) return launch_band_m<T, OP_PLANE, true>(op, g, r, xin, xout, st);
     return launch_band_m<T, OP_PLANE, false>(op, g, r, xin, xout, st);
@@ -870,10 +924,10 @@ bool launch_band_op(const LevelOp<T> &op, const Geom &g, const T *r, const T *xi
 
 }  // namespace
 
-// Where the band sweep runs: the elasticity stencil shared by every interior
-// node or a plane-invariant coarse operator, a level periodic in x and y
-// with 8, 16, 32, 64 or 128 sub-grid columns (16 .. 256 nodes) and whole
-// bands of 8 rows (at least two), an even z extent if z is periodic.  FP32 levels by default;
+// Where the band sweep runs: a shared stencil or a plane-invariant coarse
+// operator, a level periodic in x and y, rows of up to 256 nodes whose colours
+// are whole 16-byte units (the tensor maps' strides), whole bands of 8 rows
+// (at least two), an even z extent if z is periodic.  FP32 levels by default;
 // STZ_MG_BAND=0 turns it off, STZ_MG_BAND=1 uses it in FP64 too.
 template <typename T>
 bool gs_band_applies(const LevelOp<T> &op, const Geom &g) {
@@ -881,10 +935,10 @@ bool gs_band_applies(const LevelOp<T> &op, const Geom &g) {
     if (const char *e = std::getenv("STZ_MG_BAND")) mode = std::atoi(e) != 0;
     if (mode == 0) return false;
     if (mode < 0 && sizeof(T) != 4) return false;
-    if (!((op.kind == OP_CONST && op.cop.elastic) || op.kind == OP_PLANE)) return false;
+    if (op.kind != OP_CONST && op.kind != OP_PLANE) return false;
     const int rows = band_rows(g.M2);
     if (!g.xp || !g.yp || (g.m & 1) || g.n % rows != 0 || g.n < 2 * rows) return false;
-    if (g.M2 != 8 && g.M2 != 16 && g.M2 != 32 && g.M2 != 64 && g.M2 != 128) return false;
+    if (band_pad<T>(g.M2) == 0 || g.M2 * sizeof(T) % 16 != 0) return false;
     if (g.zp && (g.o & 1)) return false;
     return true;
 }
@@ -898,12 +952,12 @@ bool launch_gs_sweep_band(const LevelOp<T> &op, const Geom &g, const T *r, const
 
 namespace {
 
-template <typename T, int M2, int KIND, bool SPARSE>
+template <typename T, int M2, int KIND, bool SPARSE, bool PAD = false>
 bool launch_res_band_k(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, T *res, cudaStream_t st) {
     BandMaps xm;
-    if (!make_band_maps<T>(g, x, xm)) return false;
+    if (!make_band_maps<T>(g, M2, x, xm)) return false;
     constexpr int NH = kResNH<T, M2>;
-    auto kern = residual_band_kernel<T, M2, NH, KIND, SPARSE>;
+    auto kern = residual_band_kernel<T, M2, NH, KIND, SPARSE, PAD>;
     const int smem = kBandWords<M2> * (int)sizeof(T);
     static unsigned long long attr_devices = 0;
     if (first_band_use(attr_devices)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -920,14 +974,22 @@ bool launch_res_band_k(const LevelOp<T> &op, const Geom &g, const T *r, const T 
 
 template <typename T, int KIND, bool SPARSE>
 bool launch_res_band_m(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, T *res, cudaStream_t st) {
-    switch (g.M2) {
+    switch (band_pad<T>(g.M2)) {
         case 8: return launch_res_band_k<T, 8, KIND, SPARSE>(op, g, r, x, res, st);
         case 16: return launch_res_band_k<T, 16, KIND, SPARSE>(op, g, r, x, res, st);
         case 32: return launch_res_band_k<T, 32, KIND, SPARSE>(op, g, r, x, res, st);
         case 64: return launch_res_band_k<T, 64, KIND, SPARSE>(op, g, r, x, res, st);
-        case 128: return launch_res_band_k<T, 128, KIND, SPARSE>(op, g, r, x, res, st);
-        default: return false;
+        case 128: if (g.M2 == 128) return launch_res_band_k<T, 128, KIND, SPARSE>(op, g, r, x, res, st);
     }
+    if constexpr (sizeof(T) == 4) {
+        switch (band_pad<T>(g.M2)) {
+            case 24: return launch_res_band_k<T, 24, KIND, SPARSE, true>(op, g, r, x, res, st);
+            case 48: return launch_res_band_k<T, 48, KIND, SPARSE, true>(op, g, r, x, res, st);
+            case 96: return launch_res_band_k<T, 96, KIND, SPARSE, true>(op, g, r, x, res, st);
+            case 128: return launch_res_band_k<T, 128, KIND, SPARSE, true>(op, g, r, x, res, st);
+        }
+    }
+    return false;
 }
 
 template <typename T>
@@ -950,7 +1012,7 @@ bool launch_residual_band(const LevelOp<T> &op, const Geom &g, const T *r, const
     if (!gs_band_applies(op, g)) return false;
     int mode = -1;
     if (const char *e = std::getenv("STZ_MG_BAND_RES")) mode = std::atoi(e) != 0;
-    if (mode == 0 || (mode < 0 && op.kind != OP_PLANE)) return false;
+    if (mode == 0 || (mode < 0 && op.kind != OP_PLANE) || (op.kind == OP_CONST && !op.cop.elastic)) return false;
     return launch_res_band_op<T>(op, g, r, x, res, st);
 }
 template bool launch_residual_band<float>(const LevelOp<float> &, const Geom &, const float *, const float *, float *,
@@ -962,7 +1024,7 @@ template bool launch_residual_band<double>(const LevelOp<double> &, const Geom &
 template <typename T>
 bool gs_band_ready(const Geom &g, const T *field) {
     BandMaps mp;
-    return make_band_maps<T>(g, field, mp);
+    return make_band_maps<T>(g, band_pad<T>(g.M2), field, mp);
 }
 template bool gs_band_ready<float>(const Geom &, const float *);
 template bool gs_band_ready<double>(const Geom &, const double *);

@@ -149,6 +149,7 @@ struct ConstOp {
     T inv_fix[9];
     int elastic;
     int centre_diag;   // the centre block a[13] is diagonal
+    int corners;       // some corner block is not zero
 };
 
 // Per-node Lame coefficients (variable-mu operator, matrix-free).

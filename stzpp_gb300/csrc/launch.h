@@ -36,8 +36,9 @@ constexpr int kDensePartials = 304;   // at most
 template <typename T, typename R>
 int launch_residual_dense(const LevelOp<T> &op, const Geom &g, const T *r, const T *x, R *res, double *partial,
                           cudaStream_t st);
-// plane.cu: one FP64 sweep in place, and the residual, of a plane-invariant level
-void launch_gs_sweep_plane64(const PlaneOp<double> &op, const Geom &g, const double *r, double *x, cudaStream_t st);
+// plane.cu: one sweep in place, and the FP64 residual, of a plane-invariant level
+template <typename T>
+void launch_gs_sweep_plane(const PlaneOp<T> &op, const Geom &g, const T *r, T *x, cudaStream_t st);
 void launch_residual_plane64(const PlaneOp<double> &op, const Geom &g, const double *r, const double *x, double *res,
                              cudaStream_t st);
 // tile.cu: one sweep reading xin and writing xout (levels periodic in x, y

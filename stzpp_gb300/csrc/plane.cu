@@ -1,7 +1,9 @@
 // FP64 Gauss-Seidel sweep and residual of the plane-invariant coarse levels
-// (OP_PLANE): every node of a plane has the same row of 27 blocks.
+// (OP_PLANE), where every node of a plane has the same row of 27 blocks, and
+// the FP32 sweep of those that the bands (band.cu) do not take and that are
+// small enough to be bound by latency.
 //
-// The FP64 pipe bounds these levels: an SM scheduler issues one instruction
+// The FP64 pipe bounds the FP64 levels: an SM scheduler issues one instruction
 // every 64 cycles, with one active lane or 32, so what counts is that lanes
 // are full, that all four schedulers of every SM have warps, and the number of
 // instructions.  A lane takes one row of one node (10 nodes a warp), the
@@ -61,17 +63,17 @@ struct LaneRow {
 // acc -= blocks 9 d .. 9 d + 8 of the lane's row (d = 0, 1, 2: the planes
 // below, at and above the node), x of the node's own plane through L2 when
 // other CTAs write it (COH).
-template <bool SPARSE, bool WITH_CENTRE, bool COH>
-__device__ __forceinline__ double row_part(int d, const double *cf, const LaneRow &L, const NbrOffsets &t,
-                                           const double *x, int npad, double acc) {
-    const double *xr = x + t.oz[d];
+template <typename T, bool SPARSE, bool WITH_CENTRE, bool COH>
+__device__ __forceinline__ T row_part(int d, const T *cf, const LaneRow &L, const NbrOffsets &t, const T *x, int npad,
+                                      T acc) {
+    const T *xr = x + t.oz[d];
     const bool zin = t.oz[d] >= 0;
-    auto value = [&](const double *p, bool in) {
-        double v = 0.0;
+    auto value = [&](const T *p, bool in) {
+        T v = T(0);
         if (in) v = COH && d == 1 ? __ldcg(p) : *p;
         return v;
     };
-    double v[9][3];
+    T v[9][3];
 #pragma unroll
     for (int n = 0; n < 9; n++) {
         const int dx = n % 3 - 1, dy = n / 3 - 1, s = t.ox[dx + 1] + t.oy[dy + 1];
@@ -89,7 +91,7 @@ __device__ __forceinline__ double row_part(int d, const double *cf, const LaneRo
             for (int c = 0; c < 3; c++) v[n][c] = value(xr + s + c * (size_t)npad, in);
         }
     }
-    const double *c = cf + 81 * d + 3 * L.row;
+    const T *c = cf + 81 * d + 3 * L.row;
 #pragma unroll
     for (int n = 0; n < 9; n++) {
         const int dx = n % 3 - 1, dy = n / 3 - 1;
@@ -100,7 +102,7 @@ __device__ __forceinline__ double row_part(int d, const double *cf, const LaneRo
         } else if (SPARSE && axes == 2) {
             const int pair = d == 1 ? 0 : dx != 0 ? 1 : 2;
             acc = fma_rn(-c[9 * n + L.first[pair]], v[n][0], acc);
-            acc = fma_rn(L.two[pair] ? -c[9 * n + L.second[pair]] : -0.0, v[n][1], acc);
+            acc = fma_rn(L.two[pair] ? -c[9 * n + L.second[pair]] : T(-0.0), v[n][1], acc);
         } else {
 #pragma unroll
             for (int e = 0; e < 3; e++) acc = fma_rn(-c[9 * n + e], v[n][e], acc);
@@ -109,27 +111,29 @@ __device__ __forceinline__ double row_part(int d, const double *cf, const LaneRo
     return acc;
 }
 
-__device__ __forceinline__ void stage_row(const PlaneOp<double> &op, int k, double *cf) {
+template <typename T>
+__device__ __forceinline__ void stage_row(const PlaneOp<T> &op, int k, T *cf) {
     for (int e = threadIdx.x; e < 252; e += blockDim.x)
         cf[e] = e < 243 ? op.coef[(size_t)e * op.O + k] : op.dinv[(size_t)(e - 243) * op.O + k];
     __syncthreads();
 }
 
 // One item of a lane's row, whichever structure its plane has.
-template <bool WITH_CENTRE, bool COH>
-__device__ __forceinline__ double any_row_part(bool sparse, int d, const double *cf, const LaneRow &L,
-                                               const NbrOffsets &t, const double *x, int npad, double acc) {
-    if (sparse) return row_part<true, WITH_CENTRE, COH>(d, cf, L, t, x, npad, acc);
-    return row_part<false, WITH_CENTRE, COH>(d, cf, L, t, x, npad, acc);
+template <bool WITH_CENTRE, bool COH, typename T>
+__device__ __forceinline__ T any_row_part(bool sparse, int d, const T *cf, const LaneRow &L, const NbrOffsets &t,
+                                          const T *x, int npad, T acc) {
+    if (sparse) return row_part<T, true, WITH_CENTRE, COH>(d, cf, L, t, x, npad, acc);
+    return row_part<T, false, WITH_CENTRE, COH>(d, cf, L, t, x, npad, acc);
 }
 
 constexpr int kMaxWarps = 12;   // two CTAs share an SM: their colours' barriers overlap
 
 // Colours 4c .. 4c+3 of every plane of parity c, `cl` CTAs (one cluster) per
 // plane; x is updated in place.
+template <typename T>
 __global__ void __launch_bounds__(32 * kMaxWarps, 2)
-    gs_plane64_kernel(Geom g, int c, int cl, PlaneOp<double> op, const double *__restrict__ r, double *x) {
-    __shared__ double cf[252];
+    gs_plane_rows_kernel(Geom g, int c, int cl, PlaneOp<T> op, const T *__restrict__ r, T *x) {
+    __shared__ T cf[252];
     const int lane = threadIdx.x & 31, row = min(lane / kNodes, 2), node = lane % kNodes;
     const int rank = blockIdx.x % cl, K = blockIdx.x / cl, plane = g.M2 * g.N2;
     const int warps = cl * (blockDim.x >> 5), first = rank * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2)
     dim_offsets(K, c, g.o, g.O2, g.zp, 4 * g.S, plane, nb.oz);
     int p = -1;
     bool any = false;   // an item without nodes must not take the FP64 pipe from the others
-    double acc = 0.0;
+    T acc = T(0);
     // item n of this warp in colour q, and the blocks below its plane
     auto begin = [&](int q, int n) {
         const int t = kNodes * (first + n * warps) + node, J = t / g.M2, I = t - J * g.M2;
@@ -153,17 +157,17 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2)
         p = valid ? q * g.S + K * plane + t : -1;
         dim_offsets(valid ? I : 0, q & 1, g.m, g.M2, g.xp, g.S, 1, nb.ox);
         dim_offsets(valid ? J : 0, (q >> 1) & 1, g.n, g.N2, g.yp, 2 * g.S, g.M2, nb.oy);
-        acc = valid ? r[p + row * np] : 0.0;
+        acc = valid ? r[p + row * np] : T(0);
         acc = any_row_part<false, true>(sparse, 0, cf, L, nb, x, g.npad, acc);
     };
     auto end = [&]() {
         if (!any) return;
         acc = any_row_part<false, true>(sparse, 1, cf, L, nb, x, g.npad, acc);
         acc = any_row_part<false, true>(sparse, 2, cf, L, nb, x, g.npad, acc);
-        const double a0 = __shfl_sync(0xffffffffu, acc, node), a1 = __shfl_sync(0xffffffffu, acc, node + kNodes),
-                     a2 = __shfl_sync(0xffffffffu, acc, node + 2 * kNodes);
-        const double *inv = cf + 243 + 3 * row;
-        const double xn = dot3(inv[0], a0, inv[1], a1, inv[2], a2);
+        const T a0 = __shfl_sync(0xffffffffu, acc, node), a1 = __shfl_sync(0xffffffffu, acc, node + kNodes),
+                a2 = __shfl_sync(0xffffffffu, acc, node + 2 * kNodes);
+        const T *inv = cf + 243 + 3 * row;
+        const T xn = dot3(inv[0], a0, inv[1], a1, inv[2], a2);
         if (p >= 0) x[p + row * np] = xn;
     };
     begin(4 * c, 0);
@@ -218,7 +222,8 @@ __global__ void __launch_bounds__(256)
 // 10 nodes of a colour of the plane as far as 8 CTAs of 12 warps go, the
 // warps spread over the CTAs before they are added to them: on a small plane a
 // second warp on a scheduler only waits for the first.
-void launch_gs_sweep_plane64(const PlaneOp<double> &op, const Geom &g, const double *r, double *x, cudaStream_t st) {
+template <typename T>
+void launch_gs_sweep_plane(const PlaneOp<T> &op, const Geom &g, const T *r, T *x, cudaStream_t st) {
     const int groups = (g.M2 * g.N2 + kNodes - 1) / kNodes;
     const int cl = groups > 16 ? 8 : groups > 8 ? 4 : groups > 4 ? 2 : 1;
     const int warps = std::min(kMaxWarps, ((groups + cl - 1) / cl + 3) / 4 * 4);
@@ -235,9 +240,13 @@ void launch_gs_sweep_plane64(const PlaneOp<double> &op, const Geom &g, const dou
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, gs_plane64_kernel, g, c, cl, op, r, x);
+        cudaLaunchKernelEx(&cfg, gs_plane_rows_kernel<T>, g, c, cl, op, r, x);
     }
 }
+
+template void launch_gs_sweep_plane<float>(const PlaneOp<float> &, const Geom &, const float *, float *, cudaStream_t);
+template void launch_gs_sweep_plane<double>(const PlaneOp<double> &, const Geom &, const double *, double *,
+                                            cudaStream_t);
 
 void launch_residual_plane64(const PlaneOp<double> &op, const Geom &g, const double *r, const double *x, double *res,
                              cudaStream_t st) {

@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(kBlock) gs_plane_kernel(Geom g, int q, int rev
 // order, separated by __syncthreads, without any dependency on other blocks:
 // a full 8-colour sweep is two launches (even planes, then odd planes), with
 // the same arithmetic and the same result as eight colour launches.
-template <typename T, int KIND, bool ELASTIC, bool SPARSE>
-__device__ inline void gs_node(const LevelOp<T> &op, const Geom &g, int q, int I, int J, int K, const T *cf,
+template <typename T, int KIND, bool ELASTIC>
+__device__ inline void gs_node(const LevelOp<T> &op, const Geom &g, int q, int I, int J, int K,
                                const T *__restrict__ r, T *__restrict__ x) {
     const int i = 2 * I + (q & 1), j = 2 * J + ((q >> 1) & 1), k = 2 * K + ((q >> 2) & 1);
     if (i >= g.m || j >= g.n || k >= g.o) return;
@@ -149,7 +149,7 @@ __device__ inline void gs_node(const LevelOp<T> &op, const Geom &g, int q, int I
         }
 #pragma unroll
         for (int e = 0; e < 9; e++) inv[e] = src[e];
-    } else if (KIND == OP_LAME) {
+    } else {
         T c3[3];
         if (is_interior(g, i, j, k)) {
             lame_row<T, false>(op.lop, g, nb, p, x, acc, c3);
@@ -160,10 +160,6 @@ __device__ inline void gs_node(const LevelOp<T> &op, const Geom &g, int q, int I
         x[p + g.npad] = acc[1] / c3[1];
         x[p + 2 * g.npad] = acc[2] / c3[2];
         return;
-    } else {
-        plane_row_coef<T, SPARSE, false>(cf, 1, g, nb, x, acc);
-#pragma unroll
-        for (int e = 0; e < 9; e++) inv[e] = cf[243 + e];
     }
     x[p] = dot3(inv[0], acc[0], inv[1], acc[1], inv[2], acc[2]);
     x[p + g.npad] = dot3(inv[3], acc[0], inv[4], acc[1], inv[5], acc[2]);
@@ -172,38 +168,28 @@ __device__ inline void gs_node(const LevelOp<T> &op, const Geom &g, int q, int I
 
 constexpr int kPhaseThreads = 512;
 
-template <typename T, int KIND, bool ELASTIC, bool SPARSE>
+template <typename T, int KIND, bool ELASTIC>
 __global__ void __launch_bounds__(kPhaseThreads) gs_phase_kernel(Geom g, int c, const __grid_constant__ LevelOp<T> op,
                                                                  const T *__restrict__ r, T *__restrict__ x) {
-    __shared__ T cf[252];
     const int K = blockIdx.x;   // sub-grid plane: node plane k = 2K + c
-    if (KIND == OP_PLANE) {
-        const int k = 2 * K + c;
-        for (int e = threadIdx.x; e < 252; e += blockDim.x)
-            cf[e] = k < g.o ? (e < 243 ? op.pop.coef[e * op.pop.O + k] : op.pop.dinv[(e - 243) * op.pop.O + k]) : T(0);
-        __syncthreads();
-    }
     const int plane = g.M2 * g.N2;
     for (int qxy = 0; qxy < 4; qxy++) {
         const int q = qxy + 4 * c;
         for (int t = threadIdx.x; t < plane; t += blockDim.x) {
-            // keep the shared-memory coefficient reads inside the loop (hoisting
-            // all 243 of them into registers would spill)
-            asm volatile("" ::: "memory");
             const int J = t / g.M2, I = t - J * g.M2;
-            gs_node<T, KIND, ELASTIC, SPARSE>(op, g, q, I, J, K, cf, r, x);
+            gs_node<T, KIND, ELASTIC>(op, g, q, I, J, K, r, x);
         }
         __syncthreads();
     }
 }
 
-template <typename T, int KIND, bool ELASTIC, bool SPARSE>
+template <typename T, int KIND, bool ELASTIC>
 static void launch_phases(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cudaStream_t st) {
     const int plane = g.M2 * g.N2;
     const int threads = plane >= kPhaseThreads ? kPhaseThreads : ((plane + 31) / 32) * 32;
     const int even = (g.o + 1) / 2, odd = g.o / 2;
-    gs_phase_kernel<T, KIND, ELASTIC, SPARSE><<<even, threads, 0, st>>>(g, 0, op, r, x);
-    if (odd > 0) gs_phase_kernel<T, KIND, ELASTIC, SPARSE><<<odd, threads, 0, st>>>(g, 1, op, r, x);
+    gs_phase_kernel<T, KIND, ELASTIC><<<even, threads, 0, st>>>(g, 0, op, r, x);
+    if (odd > 0) gs_phase_kernel<T, KIND, ELASTIC><<<odd, threads, 0, st>>>(g, 1, op, r, x);
 }
 
 // ------------------------------------------------------------- residual
@@ -348,12 +334,17 @@ void launch_gs_sweeps(const LevelOp<T> &op, const Geom &g, const T *r, T *x, T *
     // plane-invariant levels of 64x64 and more: 4+ tiles per plane beat one
     // block per plane (64x64x65, two FP32 sweeps: 58 vs 107 us); 32x32 does not
     const bool plane_tiles = op.kind == OP_PLANE && g.m * g.n >= 64 * 64;
-    // the fine level of a shared elasticity stencil: full-width bands whose
-    // planes arrive by TMA (band.cu)
+    // shared stencils and plane-invariant levels: full-width bands whose planes
+    // arrive by TMA (band.cu); a last odd sweep comes back by a copy, which is
+    // a fraction of the sweep and far less than eight colour launches
     if (tmp && gs_band_applies(op, g)) {
         for (; s + 2 <= sweeps; s += 2) {
             if (!launch_gs_sweep_band(op, g, r, x, tmp, st)) break;
             launch_gs_sweep_band(op, g, r, tmp, x, st);
+        }
+        if (s + 1 == sweeps && launch_gs_sweep_band(op, g, r, x, tmp, st)) {
+            cudaMemcpyAsync(x, tmp, 3 * (size_t)g.npad * sizeof(T), cudaMemcpyDeviceToDevice, st);
+            s++;
         }
     }
     if (tmp && (large_planes(op, g) || plane_tiles) && gs_tile_applies(op, g))
@@ -380,14 +371,12 @@ void launch_gs_sweep(const LevelOp<T> &op, const Geom &g, const T *r, T *x, cuda
     }
     switch (op.kind) {
         case OP_CONST:
-            if (op.cop.elastic) launch_phases<T, OP_CONST, true, false>(op, g, r, x, st);
-            else launch_phases<T, OP_CONST, false, false>(op, g, r, x, st);
+            if (op.cop.elastic) launch_phases<T, OP_CONST, true>(op, g, r, x, st);
+            else launch_phases<T, OP_CONST, false>(op, g, r, x, st);
             break;
-        case OP_LAME: launch_phases<T, OP_LAME, false, false>(op, g, r, x, st); break;
+        case OP_LAME: launch_phases<T, OP_LAME, false>(op, g, r, x, st); break;
         case OP_PLANE:
-            if constexpr (sizeof(T) == 8) launch_gs_sweep_plane64(op.pop, g, r, x, st);
-            else if (op.pop.sparse) launch_phases<T, OP_PLANE, false, true>(op, g, r, x, st);
-            else launch_phases<T, OP_PLANE, false, false>(op, g, r, x, st);
+            launch_gs_sweep_plane<T>(op.pop, g, r, x, st);
             break;
         default: launch_gs_sweep_dense<T>(op, g, r, x, st); break;
     }
