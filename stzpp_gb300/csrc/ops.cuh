@@ -177,27 +177,37 @@ __device__ inline void lame_row64(const LameOp<double> &op, const Geom &g, const
     }
 }
 
-// acc -= sum over the 18 non-zero off-centre blocks (and the centre if asked).
-template <typename T, bool WITH_CENTRE>
-__device__ inline void lame_row(const LameOp<T> &op, const Geom &g, const NbrOffsets &t, int p,
-                                const T *__restrict__ x, T *acc, T *centre_out) {
-    if constexpr (sizeof(T) == 8) {
-        lame_row64<WITH_CENTRE>(op, g, t, p, x, acc, centre_out);
-        return;
+// acc -= sum over the 18 non-zero off-centre blocks (and the centre if asked),
+// the node's surroundings given by `at`: at.mu0, at.lam0 its coefficients,
+// at.mu(f), at.lam(f) those of its face neighbours (x-, x+, y-, y+, z-, z+) and
+// at.x(dx, dy, dz, c) the component c of a neighbour.
+template <typename T, bool WITH_CENTRE, typename N>
+__device__ __forceinline__ void lame_row_of(const LameOp<T> &op, const N &at, T *acc, T *centre_out) {
+    T mu_nb[6], lam_nb[6], face[6][3], centre[3];
+    T cen[3] = {T(0), T(0), T(0)};
+#pragma unroll
+    for (int f = 0; f < 6; f++) {
+        mu_nb[f] = at.mu(f);
+        lam_nb[f] = at.lam(f);
+        const int ax = f / 2;
+        T mu_f = T(0.5) * (at.mu0 + mu_nb[f]);
+        T lam_f = T(0.5) * (at.lam0 + lam_nb[f]);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            T v = (c == ax ? (lam_f + T(2) * mu_f) : mu_f) * op.ih2[ax];
+            face[f][c] = -op.dt * v;
+            cen[c] -= v;
+        }
     }
-    LameRow<T> L;
-    T mu_nb[6], lam_nb[6];
-    lame_faces(op, g, t, p, L, mu_nb, lam_nb);
-    const int npad = g.npad;
+#pragma unroll
+    for (int c = 0; c < 3; c++) centre[c] = -op.dt * cen[c];
     // faces
 #pragma unroll
     for (int f = 0; f < 6; f++) {
-        const int ax = f / 2, s = (f & 1) ? 2 : 0;
-        int sl = (ax == 0 ? t.ox[s] : t.ox[1]) + (ax == 1 ? t.oy[s] : t.oy[1]) + (ax == 2 ? t.oz[s] : t.oz[1]);
-        T v[3];
-        load3(x, npad, sl, v);
+        const int ax = f / 2, d = f & 1 ? 1 : -1;
 #pragma unroll
-        for (int c = 0; c < 3; c++) acc[c] -= L.face[f][c] * v[c];
+        for (int c = 0; c < 3; c++)
+            acc[c] -= face[f][c] * at.x(ax == 0 ? d : 0, ax == 1 ? d : 0, ax == 2 ? d : 0, c);
     }
     // edges: component pair (r, c) in the plane of axes (r, c)
 #pragma unroll
@@ -211,27 +221,49 @@ __device__ inline void lame_row(const LameOp<T> &op, const Geom &g, const NbrOff
                 int d[3] = {0, 0, 0};
                 d[r] = sr;
                 d[c] = sc;
-                int sl = t.ox[d[0] + 1] + t.oy[d[1] + 1] + t.oz[d[2] + 1];
                 const T sgn = T(sr * sc);
                 // neighbour coefficient values: lam/mu at p + sr e_r and p + sc e_c
                 const T lam_r = lam_nb[2 * r + (sr > 0)], mu_r = mu_nb[2 * r + (sr > 0)];
                 const T lam_c = lam_nb[2 * c + (sc > 0)], mu_c = mu_nb[2 * c + (sc > 0)];
                 const T a_rc = -op.dt * ((sgn * (lam_r + mu_c)) * ie);
                 const T a_cr = -op.dt * ((sgn * (lam_c + mu_r)) * ie);
-                acc[r] -= a_rc * x[sl + c * npad];
-                acc[c] -= a_cr * x[sl + r * npad];
+                acc[r] -= a_rc * at.x(d[0], d[1], d[2], c);
+                acc[c] -= a_cr * at.x(d[0], d[1], d[2], r);
             }
     }
-    if (WITH_CENTRE) {
-        T v[3];
-        load3(x, npad, p, v);
 #pragma unroll
-        for (int c = 0; c < 3; c++) acc[c] -= L.centre[c] * v[c];
+    for (int c = 0; c < 3; c++) {
+        if (WITH_CENTRE) acc[c] -= centre[c] * at.x(0, 0, 0, c);
+        if (centre_out) centre_out[c] = centre[c];
     }
-    if (centre_out) {
-#pragma unroll
-        for (int c = 0; c < 3; c++) centre_out[c] = L.centre[c];
+}
+
+// The surroundings in the level's fields.
+template <typename T>
+struct LameNode {
+    const LameOp<T> &op;
+    const NbrOffsets &t;
+    const T *x_;
+    int npad;
+    T mu0, lam0;
+    __device__ __forceinline__ LameNode(const LameOp<T> &op, const Geom &g, const NbrOffsets &t, int p, const T *x)
+        : op(op), t(t), x_(x), npad(g.npad), mu0(op.mu[p]), lam0(op.lam[p]) {}
+    __device__ __forceinline__ int face(int f) const {
+        const int s = f & 1 ? 2 : 0;
+        return t.ox[f / 2 == 0 ? s : 1] + t.oy[f / 2 == 1 ? s : 1] + t.oz[f / 2 == 2 ? s : 1];
     }
+    __device__ __forceinline__ T mu(int f) const { return op.mu[face(f)]; }
+    __device__ __forceinline__ T lam(int f) const { return op.lam[face(f)]; }
+    __device__ __forceinline__ T x(int dx, int dy, int dz, int c) const {
+        return x_[t.ox[dx + 1] + t.oy[dy + 1] + t.oz[dz + 1] + c * npad];
+    }
+};
+
+template <typename T, bool WITH_CENTRE>
+__device__ inline void lame_row(const LameOp<T> &op, const Geom &g, const NbrOffsets &t, int p,
+                                const T *__restrict__ x, T *acc, T *centre_out) {
+    if constexpr (sizeof(T) == 8) lame_row64<WITH_CENTRE>(op, g, t, p, x, acc, centre_out);
+    else lame_row_of<T, WITH_CENTRE>(op, LameNode<T>(op, g, t, p, x), acc, centre_out);
 }
 
 template <typename T>
