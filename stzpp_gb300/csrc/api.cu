@@ -718,9 +718,10 @@ void enqueue_vcycle(stz_mg_handle h, Hier<T> H) {
                             h->st);
         if (!launch_residual_restrict<T>(H.op[i], g, h->geo[i + 1], H.L[i].r, H.L[i].x, H.L[i + 1].r, h->st)) {
             launch_residual<T, T>(H.op[i], g, H.L[i].r, H.L[i].x, H.L[i].res, nullptr, nullptr, h->st);
-            launch_restriction<T>(g, h->geo[i + 1], H.L[i].res, H.L[i + 1].r, h->st);
+            launch_restriction<T>(g, h->geo[i + 1], H.L[i].res, H.L[i + 1].r, H.L[i + 1].x, h->st);
+        } else {
+            CK(cudaMemsetAsync(H.L[i + 1].x, 0, 3 * (size_t)h->geo[i + 1].npad * sizeof(T), h->st));
         }
-        CK(cudaMemsetAsync(H.L[i + 1].x, 0, 3 * (size_t)h->geo[i + 1].npad * sizeof(T), h->st));
     }
     TailDesc<T> td{};
     if (h->tail_lo >= 0) {
@@ -1472,7 +1473,7 @@ int stz_mg_level_restrict_residual(stz_mg_handle h, int level) {
         check_level(h, level);
         if (level < 1) fail(STZ_MG_ERR_ARG, "restriction target must be a coarse level");
         const int f = level - 1;
-        launch_restriction<double>(h->geo[f], h->geo[level], h->L64[f].res, h->L64[level].r, h->st);
+        launch_restriction<double>(h->geo[f], h->geo[level], h->L64[f].res, h->L64[level].r, nullptr, h->st);
         CK(cudaMemsetAsync(h->L64[level].x, 0, 3 * (size_t)h->geo[level].npad * sizeof(double), h->st));
         check_launch();
         sync(h);
@@ -1500,7 +1501,7 @@ int stz_mg_level_restriction(stz_mg_handle h, int level) {
         const int f = level - 1;
         launch_residual<double, double>(h->op64[f], h->geo[f], h->L64[f].r, h->L64[f].x, h->L64[f].res, nullptr,
                                         nullptr, h->st);
-        launch_restriction<double>(h->geo[f], h->geo[level], h->L64[f].res, h->L64[level].r, h->st);
+        launch_restriction<double>(h->geo[f], h->geo[level], h->L64[f].res, h->L64[level].r, nullptr, h->st);
         CK(cudaMemsetAsync(h->L64[level].x, 0, 3 * (size_t)h->geo[level].npad * sizeof(double), h->st));
         sync(h);
     });
@@ -1624,8 +1625,8 @@ int stz_mg_time_kernel(stz_mg_handle h, int kernel, int level, int reps, double 
                 if (level < 1) fail(STZ_MG_ERR_ARG, "restriction target must be a coarse level");
                 const Geom &gf = h->geo[level - 1];
                 work = 3 * s * ((double)npts(gf) + npts_l);
-                if (mixed) launch = [&] { launch_restriction<float>(gf, g, h->L32[level - 1].res, h->L32[level].r, h->st); };
-                else launch = [&] { launch_restriction<double>(gf, g, h->L64[level - 1].res, h->L64[level].r, h->st); };
+                if (mixed) launch = [&] { launch_restriction<float>(gf, g, h->L32[level - 1].res, h->L32[level].r, nullptr, h->st); };
+                else launch = [&] { launch_restriction<double>(gf, g, h->L64[level - 1].res, h->L64[level].r, nullptr, h->st); };
                 break;
             }
             case STZ_MG_K_INTERP: {

@@ -135,6 +135,14 @@ struct BandMaps {
     CUtensorMap full, less1, one;
 };
 
+// The maps into the descriptor cache, ahead of their first use.
+__device__ __forceinline__ void prefetch_maps(const BandMaps &mp) {
+    const CUtensorMap *maps[3] = {&mp.full, &mp.less1, &mp.one};
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<unsigned long long>(maps[i])) : "memory");
+}
+
 struct BandArgs {
     Geom g;
     int c;          // plane parity of this launch
@@ -246,7 +254,9 @@ __device__ __forceinline__ void band_colour(const T *__restrict__ s, const int (
             constexpr int dx = bxy % 3 - 1, dy = bxy / 3 - 1;
             constexpr int ap = (A + dx + 2) & 1, sI = (A + dx + 2) / 2 - 1;
             constexpr int bp = (B + dy + 2) & 1, sJ = (B + dy + 2) / 2 - 1;
-            asm volatile("" ::: "memory");
+            // with several rows a thread has enough to do between two loads;
+            // with one the loads of a plane's nine blocks go out together
+            if constexpr (NR > 1) asm volatile("" ::: "memory");
             T cb[kCoefPad];
             load_block_coef<T>(cf + kCoefPad * b, cb);
 #pragma unroll
@@ -466,7 +476,6 @@ __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp
             r3[u][cc] = __ldcs(r + s3 + cc * np);
         }
     }
-    if (KIND == OP_PLANE) stage_coef<T>(op.pop, k, cfs, tid, NH * M2);   // plane k's row of coefficients
     const bool ok = mbar_wait(bar, phase, 200000000ull);   // 0.2 s: copies that never arrive
     if (!__syncthreads_and(ok)) {
         if (tid == 0) {
@@ -531,6 +540,7 @@ __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp
         emit(I0{}, I1{}, NR1{}, t0b, nb, o, true);
     }
     __syncthreads();
+    chain_next();
     {
         T o[P1][3];
         band_colour<T, M2, KIND, SPARSE, 1, 1, P1>(s, ibb, op, cfs, nb, r3, o);
@@ -557,20 +567,26 @@ __global__ void __launch_bounds__(NH * M2, (kBandMinBlocks<T, M2, KIND>))
     const int tid = threadIdx.x;
     const BandItem it = band_item<M2>(args, blockIdx.x);
     if (!band_stages<KIND>(it)) {
+        chain_wait();
         band_plate<T, M2, NH, PAD>(args.g, op.cop, it, args.c, r, xout);
         return;
     }
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(band_smem);
     const unsigned bar = (unsigned)__cvta_generic_to_shared(&bar_store);
     if ((sbase & 127u) != 0) {   // TMA boxes land at 128-byte aligned shared addresses only
+        chain_wait();
         if (tid == 0) atomicExch(&g_band_err, 2);
         return;
     }
     if (tid == 0) {
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        prefetch_maps(in);
+        prefetch_maps(out_maps);
     }
+    if (KIND == OP_PLANE) stage_coef<T>(op.pop, it.k, cfs, tid, NH * M2);   // plane k's row of coefficients
     __syncthreads();
+    chain_wait();
     if (tid == 0) band_issue<T, M2>(args, in, out_maps, it, sbase, bar);
     band_compute<T, M2, NH, KIND, SPARSE, PAD>(args, op, it, reinterpret_cast<T *>(band_smem), cfs, bar, 0, r, xout);
 }
@@ -697,6 +713,7 @@ __global__ void __launch_bounds__(NH * M2)
     const int tid = threadIdx.x, I = tid % M2, hh = tid / M2;
     const BandItem it = band_item<M2>(args, blockIdx.x);
     if (!it.zin) {   // a Dirichlet plate: x = r / fix
+        chain_wait();
         const size_t np = (size_t)g.npad;
         for (int w = hh; w < 4 * kOwnSub<M2> && I < g.M2; w += NH) {
             const size_t sl = band_slot(g, w / kOwnSub<M2>, args.c, it.K, it.J0 + w % kOwnSub<M2>, I);
@@ -708,14 +725,20 @@ __global__ void __launch_bounds__(NH * M2)
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(band_smem);
     const unsigned bar = (unsigned)__cvta_generic_to_shared(&bar_store);
     if ((sbase & 127u) != 0) {
+        chain_wait();
         if (tid == 0) atomicExch(&g_band_err, 2);
         return;
     }
     if (tid == 0) {
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        prefetch_maps(in);
+        prefetch_maps(out_maps);
+        prefetch_maps(mu);
+        prefetch_maps(lam);
     }
     __syncthreads();
+    chain_wait();
     if (tid == 0) {
         // an inner plane has both neighbours (a Dirichlet z ends at the plates)
         mbar_expect_tx(bar, kLameWords<M2> * (unsigned)sizeof(float));
@@ -747,6 +770,7 @@ __global__ void __launch_bounds__(NH * M2)
     __syncthreads();
     lame_colour<M2, NH, 0, 1>(args, op, it, s, ib, I, hh, r2, xout);
     __syncthreads();
+    chain_next();
     lame_colour<M2, NH, 1, 1>(args, op, it, s, ib, I, hh, r3, xout);
 }
 
@@ -883,6 +907,7 @@ __global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 96 ? 2 : 1)
     const size_t np = (size_t)g.npad;
     const bool has_lo = g.zp || k > 0, has_hi = g.zp || k < g.o - 1;
     if (KIND == OP_CONST && !(has_lo && has_hi)) {   // a Dirichlet plate: r - fix x
+        chain_wait();
 #pragma unroll 1
         for (int w = hh; w < 4 * kOwnSub<M2> && (!PAD || I < g.M2); w += NH) {
             const int ab = w / kOwnSub<M2>, t = w % kOwnSub<M2>;
@@ -900,14 +925,18 @@ __global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 96 ? 2 : 1)
     const unsigned sbase = (unsigned)__cvta_generic_to_shared(band_smem);
     const unsigned bar = (unsigned)__cvta_generic_to_shared(&bar_store);
     if ((sbase & 127u) != 0) {
+        chain_wait();
         if (tid == 0) atomicExch(&g_band_err, 2);
         return;
     }
     if (tid == 0) {
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        prefetch_maps(xm);
     }
+    if (KIND == OP_PLANE) stage_coef<T>(op.pop, k, cfs, tid, NH * M2);
     __syncthreads();
+    chain_wait();
     if (tid == 0) {
         const unsigned plane_bytes = (unsigned)(kBandWords<M2> / 3 * sizeof(T));
         mbar_expect_tx(bar, plane_bytes * (1u + has_lo + has_hi));
@@ -916,7 +945,6 @@ __global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 96 ? 2 : 1)
         stage_plane<T, M2>(xm, g, k, J0, 1, sbase, bar);
         if (has_hi) stage_plane<T, M2>(xm, g, khi, J0, 2, sbase, bar);
     }
-    if (KIND == OP_PLANE) stage_coef<T>(op.pop, k, cfs, tid, NH * M2);
     const bool ok = mbar_wait(bar, 0, 200000000ull);
     if (!__syncthreads_and(ok)) {
         if (tid == 0) {
@@ -944,6 +972,7 @@ __global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 96 ? 2 : 1)
     // scheduler would start every colour's shared loads at once
 #pragma unroll 1
     for (int q = 0; q < 4; q++) {
+        if (q == 3) chain_next();
         switch (q) {
             case 0: band_res_colour<T, M2, KIND, SPARSE, 0, 0, P>(s, ib, op, cfs, t0, nv, g, c, K, J0, I, r, res); break;
             case 1: band_res_colour<T, M2, KIND, SPARSE, 1, 0, P>(s, ib, op, cfs, t0, nv, g, c, K, J0, I, r, res); break;
@@ -1038,7 +1067,7 @@ bool launch_band_kn(const LevelOp<T> &op, const Geom &g, const T *r, const T *xi
         // first planes (and the even planes they read) are still in L2; the
         // next sweep's even launch starts at the bottom, where this one ends
         a.rev = c;
-        kern<<<a.nbands * planes, NH * M2, smem, st>>>(a, op, min_, mout, r, xout);
+        launch_chained(kern, a.nbands * planes, NH * M2, smem, st, 1, a, op, min_, mout, r, xout);
     }
     return true;
 }
@@ -1113,7 +1142,7 @@ bool launch_band_lame_m(const LameOp<float> &op, const Geom &g, const float *r, 
         a.c = c;
         a.nplanes = planes;
         a.rev = c;
-        kern<<<a.nbands * planes, NH * M2, smem, st>>>(a, op, min_, mout, mu, lam, r, xout);
+        launch_chained(kern, a.nbands * planes, NH * M2, smem, st, 1, a, op, min_, mout, mu, lam, r, xout);
     }
     return true;
 }
@@ -1190,7 +1219,7 @@ bool launch_res_band_k(const LevelOp<T> &op, const Geom &g, const T *r, const T 
     a.nplanes = g.o;
     a.rev = 0;
     a.xz = x;
-    kern<<<a.nbands * g.o, NH * M2, smem, st>>>(a, op, xm, r, res);
+    launch_chained(kern, a.nbands * g.o, NH * M2, smem, st, 1, a, op, xm, r, res);
     return true;
 }
 

@@ -139,22 +139,24 @@ __global__ void __launch_bounds__(kThreads32, 2)
     NbrOffsets nb;
     z_offsets(g, K, 4 * c, nb);
     // 32 nodes of colour q of the plane: all that may be read before the colour begins (first) or in it
-    auto load = [&](int q, bool first) {
+    auto load = [&](int q, bool first, bool chained = false) {
         const bool valid = at.t < plane && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n;
         const int s = valid ? q * g.S + K * plane + at.t : 0;
         if (!sums) {
             plane_offsets(g, at.I, at.J, q, nb);
             row.load(op, wid, s, nb, valid);
+            if (chained) chain_wait();
             if (!inplane || !first) row.load_x<true>(x, g.npad);
         } else {
             p = valid ? s : -1;
-            load3(r, g.npad, s, acc);
 #pragma unroll
             for (int e = 0; e < 9; e++) inv[e] = __ldg(op.dinv + dinv_at(s) + e * kCoefGroup);
+            if (chained) chain_wait();
+            load3(r, g.npad, s, acc);
         }
     };
     int buf = 0;
-    load(4 * c, true);
+    load(4 * c, true, true);
 #pragma unroll 1
     for (int q = 4 * c; q < 4 * c + 4; q++) {
 #pragma unroll 1
@@ -162,6 +164,7 @@ __global__ void __launch_bounds__(kThreads32, 2)
             const bool last = n + 1 == per;
             if (last) at = start;
             else at.next(g);
+            if (last && q == 4 * c + 3) chain_next();
             if (!sums) {
                 if (inplane && n == 0) row.load_x<true>(x, g.npad);
                 row.dots(wid, lane, dots[buf]);
@@ -207,7 +210,7 @@ __global__ void __launch_bounds__(kThreads32)
     int p = -1;
     bool valid = false;
     double sq = 0.0;
-    auto load = [&]() {
+    auto load = [&](bool chained = false) {
         valid = at.t < g.S && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n && 2 * at.K + (q >> 2) < g.o;
         const int s = valid ? q * g.S + at.t : 0;
         if (!sums) {
@@ -215,19 +218,23 @@ __global__ void __launch_bounds__(kThreads32)
             plane_offsets(g, at.I, at.J, q, nb);
             z_offsets(g, at.K, q, nb);
             row.load(op, wid, s, nb, valid);
+            if (chained) chain_wait();
             row.load_x<false>(x, g.npad);
         } else {
             p = at.t < g.S ? q * g.S + at.t : -1;
-            load3(r, g.npad, s, acc);
-            load3(x, g.npad, s, v);
 #pragma unroll
             for (int e = 0; e < 9; e++) cen[e] = __ldg(op.coef + coef_at(s) + (117 + e) * kCoefGroup);
+            if (chained) chain_wait();
+            load3(r, g.npad, s, acc);
+            load3(x, g.npad, s, v);
         }
     };
-    if (t0 < g.S) load();
+    if (t0 < g.S) load(true);
+    else chain_wait();
     int buf = 0;
     for (int t = t0; t < g.S; t += step, buf ^= 1) {
         const bool more = t + step < g.S;
+        if (!more) chain_next();
         if (!sums) {
             row.dots(wid, lane, dots[buf]);
             at.next(g);
@@ -348,14 +355,18 @@ __global__ void __launch_bounds__(kThreads64)
     NbrOffsets nb;
     z_offsets(g, K, 4 * c, nb);
     // 10 nodes of colour q of the plane: all that may be read before the colour begins (first) or in it
-    auto load = [&](int q, bool first, bool mine) {
+    auto load = [&](int q, bool first, bool mine, bool chained = false) {
         const bool valid =
             row < 3 && at.t < plane && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n;
         any = __any_sync(0xffffffffu, valid);
-        if (!any) return;
+        if (!any) {
+            if (chained) chain_wait();
+            return;
+        }
         const int s = valid ? q * g.S + K * plane + at.t : 0;
         plane_offsets(g, at.I, at.J, q, nb);
         rp.load<false>(op, valid, part, row < 3 ? row : 0, nb, s);
+        if (chained) chain_wait();
         if (first) rp.load_x<true, false, true>(x, g.npad, part);
         else rp.load_x<true, true, true>(x, g.npad, part);
         p = valid ? s : -1;
@@ -366,11 +377,12 @@ __global__ void __launch_bounds__(kThreads64)
         }
     };
     int w = 0;   // items so far: the warps take turns at the sums
-    load(4 * c, true, part == 0);
+    load(4 * c, true, part == 0, true);
 #pragma unroll 1
     for (int q = 4 * c; q < 4 * c + 4; q++) {
 #pragma unroll 1
         for (int n = 0; n < per; n++, w++) {
+            if (n + 1 == per && q == 4 * c + 3) chain_next();
             if (any) {   // the same for the whole team
                 if (n == 0) rp.load_x<true, true, false>(x, g.npad, part);
                 parts[team][w & 1][part][lane] = rp.sum();
@@ -413,7 +425,7 @@ __global__ void __launch_bounds__(kThreads64)
     double acc = 0.0, sq = 0.0;
     int p = -1;
     bool valid = false;
-    auto load = [&](bool mine) {
+    auto load = [&](bool mine, bool chained = false) {
         valid = row < 3 && at.t < g.S && 2 * at.I + (q & 1) < g.m && 2 * at.J + ((q >> 1) & 1) < g.n &&
                 2 * at.K + (q >> 2) < g.o;
         const int s = valid ? q * g.S + at.t : 0;
@@ -421,12 +433,15 @@ __global__ void __launch_bounds__(kThreads64)
         plane_offsets(g, at.I, at.J, q, nb);
         z_offsets(g, at.K, q, nb);
         rp.load<true>(op, valid, part, row < 3 ? row : 0, nb, s);
+        if (chained) chain_wait();
         rp.load_x<false, true, true>(x, g.npad, part);
         p = row < 3 && at.t < g.S ? q * g.S + at.t : -1;
         acc = valid && mine ? r[s + row * np] : 0.0;
     };
-    if (t0 < g.S) load(part == 0);
+    if (t0 < g.S) load(part == 0, true);
+    else chain_wait();
     for (int t = t0, n = 0; t < g.S; t += step, n++) {
+        if (t + step >= g.S) chain_next();
         parts[team][n & 1][part][lane] = rp.sum();
         team_barrier(team);
         if ((n & 3) == part) {
@@ -452,23 +467,6 @@ __global__ void __launch_bounds__(kThreads64)
     }
 }
 
-// Launches one parity of planes, `cl` CTAs (one cluster) per plane.
-template <typename T, typename K>
-void launch_planes(K kernel, int threads, int cl, int planes, const Geom &g, int c, const DenseOp<T> &op, const T *r,
-                   T *x, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(cl * planes);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, g, c, cl, op, r, x);
-}
-
 }  // namespace
 
 // One sweep of a level with per-node rows, two launches; the z extent is not
@@ -482,8 +480,10 @@ void launch_gs_sweep_dense(const LevelOp<T> &op, const Geom &g, const T *r, T *x
     for (int c = 0; c < 2; c++) {
         const int planes = c == 0 ? (g.o + 1) / 2 : g.o / 2;
         if (planes == 0) continue;
-        if constexpr (sizeof(T) == 4) launch_planes(gs_dense32_kernel, kThreads32, cl, planes, g, c, op.dop, r, x, st);
-        else launch_planes(gs_dense64_kernel, kThreads64, cl, planes, g, c, op.dop, r, x, st);
+        if constexpr (sizeof(T) == 4)
+            launch_chained(gs_dense32_kernel, cl * planes, kThreads32, 0, st, cl, g, c, cl, op.dop, r, x);
+        else
+            launch_chained(gs_dense64_kernel, cl * planes, kThreads64, 0, st, cl, g, c, cl, op.dop, r, x);
     }
 }
 
@@ -497,14 +497,16 @@ int launch_residual_dense(const LevelOp<T> &op, const Geom &g, const T *r, const
     static_assert(kDensePartials >= 8 * 38);
     if constexpr (sizeof(T) == 4) {
         const int grid = 8 * std::min((g.S + 31) / 32, 38);
-        if (partial) residual_dense32_kernel<true><<<grid, kThreads32, 0, st>>>(g, op.dop, r, x, res, partial);
-        else residual_dense32_kernel<false><<<grid, kThreads32, 0, st>>>(g, op.dop, r, x, res, nullptr);
+        if (partial) launch_chained(residual_dense32_kernel<true>, grid, kThreads32, 0, st, 1, g, op.dop, r, x, res, partial);
+        else launch_chained(residual_dense32_kernel<false>, grid, kThreads32, 0, st, 1, g, op.dop, r, x, res, nullptr);
         return grid;
     } else {
         const int items = (g.S + kNodes64 - 1) / kNodes64;
         const int grid = 8 * std::min((items + kTeams - 1) / kTeams, 19);
-        if (partial) residual_dense64_kernel<R, true><<<grid, kThreads64, 0, st>>>(g, op.dop, r, x, res, partial);
-        else residual_dense64_kernel<R, false><<<grid, kThreads64, 0, st>>>(g, op.dop, r, x, res, nullptr);
+        if (partial)
+            launch_chained(residual_dense64_kernel<R, true>, grid, kThreads64, 0, st, 1, g, op.dop, r, x, res, partial);
+        else
+            launch_chained(residual_dense64_kernel<R, false>, grid, kThreads64, 0, st, 1, g, op.dop, r, x, res, nullptr);
         return grid;
     }
 }

@@ -9,6 +9,27 @@ namespace stzmg {
 
 constexpr int kMaxLevels = 16;
 
+// A launch that may overlap the end of the one before it in the stream: of
+// kernels that call chain_wait (common.cuh), in clusters of `cluster` CTAs.
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
+                           A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // One level's operator as the kernels see it.
 template <typename T>
 struct LevelOp {
@@ -110,8 +131,9 @@ void launch_residual(const LevelOp<T> &op, const Geom &g, const T *r, const T *x
                      double *out, cudaStream_t st);
 
 // transfer.cu
+// (x_c, where not null, is cleared)
 template <typename T>
-void launch_restriction(const Geom &gf, const Geom &gc, const T *res_f, T *r_c, cudaStream_t st);
+void launch_restriction(const Geom &gf, const Geom &gc, const T *res_f, T *r_c, T *x_c, cudaStream_t st);
 template <typename T>
 void launch_interpolation(const Geom &gf, const Geom &gc, const T *x_c, T *x_f, cudaStream_t st);
 // natural-order AoS vec3 (double) <-> colour-blocked SoA

@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2)
     const LaneRow L(row);
     const bool sparse = op.structured[2 * K + c];
     stage_row(op, 2 * K + c, cf);
+    chain_wait();
     NbrOffsets nb;
     dim_offsets(K, c, g.o, g.O2, g.zp, 4 * g.S, plane, nb.oz);
     int p = -1;
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2)
     for (int q = 4 * c; q < 4 * c + 4; q++) {
 #pragma unroll 1
         for (int n = 0; n < rounds; n++) {
+            if (n + 1 == rounds && q == 4 * c + 3) chain_next();
             end();
             if (n + 1 < rounds) begin(q, n + 1);
         }
@@ -196,6 +198,7 @@ __global__ void __launch_bounds__(256)
     const int item = blockIdx.x * 8 + (threadIdx.x >> 5);
     const size_t np = (size_t)g.npad;
     if (k < g.o) stage_row(op, k, cf);
+    chain_wait();
     if (item >= 4 * groups) return;
     const int ab = item & 3, q = 4 * c + ab, t = kNodes * (item >> 2) + node, J = t / g.M2, I = t - J * g.M2;
     const bool slot = lane < 3 * kNodes && t < plane;
@@ -213,6 +216,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int d = 0; d < 3; d++) acc = any_row_part<true, false>(sparse, d, cf, L, nb, x, g.npad, acc);
     }
+    chain_next();
     if (slot) res[p + row * np] = valid ? acc : 0.0;
 }
 
@@ -230,17 +234,7 @@ void launch_gs_sweep_plane(const PlaneOp<T> &op, const Geom &g, const T *r, T *x
     for (int c = 0; c < 2; c++) {
         const int planes = c == 0 ? (g.o + 1) / 2 : g.o / 2;
         if (planes == 0) continue;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(cl * planes);
-        cfg.blockDim = dim3(32 * warps);
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cl;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, gs_plane_rows_kernel<T>, g, c, cl, op, r, x);
+        launch_chained(gs_plane_rows_kernel<T>, cl * planes, 32 * warps, 0, st, cl, g, c, cl, op, r, x);
     }
 }
 
@@ -252,7 +246,7 @@ void launch_residual_plane64(const PlaneOp<double> &op, const Geom &g, const dou
                              cudaStream_t st) {
     const int groups = (g.M2 * g.N2 + kNodes - 1) / kNodes;
     const dim3 grid((4 * groups + 7) / 8, 2 * g.O2);
-    residual_plane64_kernel<<<grid, 256, 0, st>>>(g, op, r, x, res);
+    launch_chained(residual_plane64_kernel, grid, 256, 0, st, 1, g, op, r, x, res);
 }
 
 }  // namespace stzmg

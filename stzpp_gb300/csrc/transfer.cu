@@ -28,7 +28,8 @@ __device__ inline bool regular_dim(int I, int mc, int mf, int prd) {
 }
 
 template <typename T>
-__global__ void restriction_kernel(Geom gf, Geom gc, const T *__restrict__ res, T *__restrict__ rc) {
+__global__ void restriction_kernel(Geom gf, Geom gc, const T *__restrict__ res, T *__restrict__ rc, T *__restrict__ xc) {
+    chain_wait();
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y, K = blockIdx.z;
     if (I >= gc.m || J >= gc.n) return;
     const int p = slot(gc, I, J, K);
@@ -58,9 +59,11 @@ __global__ void restriction_kernel(Geom gf, Geom gc, const T *__restrict__ res, 
     } else {
         restrict_node<T>(gf, gc, res, p, I, J, K, acc);
     }
+    chain_next();
     rc[p] = acc[0];
     rc[p + gc.npad] = acc[1];
     rc[p + 2 * gc.npad] = acc[2];
+    if (xc) xc[p] = xc[p + gc.npad] = xc[p + 2 * gc.npad] = T(0);
 }
 
 // Interpolation, one thread per coarse cell (ci,cj,ck): the cell's 8 corner
@@ -69,6 +72,7 @@ __global__ void restriction_kernel(Geom gf, Geom gc, const T *__restrict__ res, 
 // cell (c = f >> 1).
 template <typename T>
 __global__ void interpolation_kernel(Geom gf, Geom gc, const T *__restrict__ xc, T *__restrict__ xf) {
+    chain_wait();
     const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y, ck = blockIdx.z;
     if (ci >= gc.m || cj >= gc.n) return;
     const int c[3] = {ci, cj, ck}, mc[3] = {gc.m, gc.n, gc.o}, mf[3] = {gf.m, gf.n, gf.o},
@@ -111,6 +115,7 @@ __global__ void interpolation_kernel(Geom gf, Geom gc, const T *__restrict__ xc,
                 fp[sz][sy][sx] = here ? slot(gf, 2 * ci + sx, 2 * cj + sy, 2 * ck + sz) : -1;
                 if (here) load3(xf, gf.npad, fp[sz][sy][sx], f[sz][sy][sx]);
             }
+    chain_next();
 #pragma unroll
     for (int sz = 0; sz < 2; sz++) {
 #pragma unroll
@@ -235,6 +240,7 @@ __global__ void __launch_bounds__(32 * kBottomRows)
     bottom_direct_kernel(int nrow, const double *__restrict__ ainv, const int *__restrict__ nat_slot, int npad,
                          const T *__restrict__ r, T *__restrict__ x) {
     extern __shared__ double rn[];
+    chain_wait();
     const int lane = threadIdx.x & 31, row = blockIdx.x * kBottomRows + (threadIdx.x >> 5);
 #pragma unroll 4
     for (int col = threadIdx.x; col < nrow; col += 32 * kBottomRows) rn[col] = widen(r[nat_slot[col / 3] + (col % 3) * npad]);
@@ -244,6 +250,7 @@ __global__ void __launch_bounds__(32 * kBottomRows)
     const double *a = ainv + (size_t)row * nrow;
 #pragma unroll 16
     for (int col = lane; col < nrow; col += 32) acc += a[col] * rn[col];
+    chain_next();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if (lane == 0) x[nat_slot[row / 3] + (row % 3) * npad] = (T)acc;
@@ -256,14 +263,14 @@ static inline unsigned grid_stride_blocks(size_t n) {
 }
 
 template <typename T>
-void launch_restriction(const Geom &gf, const Geom &gc, const T *res_f, T *r_c, cudaStream_t st) {
+void launch_restriction(const Geom &gf, const Geom &gc, const T *res_f, T *r_c, T *x_c, cudaStream_t st) {
     dim3 blk(32, 8), grd((gc.m + 31) / 32, (gc.n + 7) / 8, gc.o);
-    restriction_kernel<T><<<grd, blk, 0, st>>>(gf, gc, res_f, r_c);
+    launch_chained(restriction_kernel<T>, grd, blk, 0, st, 1, gf, gc, res_f, r_c, x_c);
 }
 template <typename T>
 void launch_interpolation(const Geom &gf, const Geom &gc, const T *x_c, T *x_f, cudaStream_t st) {
     dim3 blk(32, 8), grd((gc.m + 31) / 32, (gc.n + 7) / 8, gc.o);
-    interpolation_kernel<T><<<grd, blk, 0, st>>>(gf, gc, x_c, x_f);
+    launch_chained(interpolation_kernel<T>, grd, blk, 0, st, 1, gf, gc, x_c, x_f);
 }
 template <typename T>
 void launch_nat_to_cb(const Geom &g, const double *nat, T *cb, cudaStream_t st) {
@@ -298,12 +305,12 @@ void launch_bottom_direct(int nrow, const double *ainv_t, const int *nat_slot, i
     const int smem = nrow * (int)sizeof(double);   // 96 KB at the 4096 nodes a direct bottom may have
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(bottom_direct_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    bottom_direct_kernel<T><<<(nrow + kBottomRows - 1) / kBottomRows, 32 * kBottomRows, smem, st>>>(nrow, ainv_t, nat_slot,
-                                                                                                  npad, r, x);
+    launch_chained(bottom_direct_kernel<T>, (nrow + kBottomRows - 1) / kBottomRows, 32 * kBottomRows, smem, st, 1, nrow,
+                   ainv_t, nat_slot, npad, r, x);
 }
 
-template void launch_restriction<float>(const Geom &, const Geom &, const float *, float *, cudaStream_t);
-template void launch_restriction<double>(const Geom &, const Geom &, const double *, double *, cudaStream_t);
+template void launch_restriction<float>(const Geom &, const Geom &, const float *, float *, float *, cudaStream_t);
+template void launch_restriction<double>(const Geom &, const Geom &, const double *, double *, double *, cudaStream_t);
 template void launch_interpolation<float>(const Geom &, const Geom &, const float *, float *, cudaStream_t);
 template void launch_interpolation<double>(const Geom &, const Geom &, const double *, double *, cudaStream_t);
 template void launch_nat_to_cb<float>(const Geom &, const double *, float *, cudaStream_t);
