@@ -13,12 +13,15 @@
 //    row, to the others, so one cluster barrier a column is enough.
 //  * gj_rows_kernel: the row swaps on the other columns; the pivot rows'
 //    values go to a w x n scratch.
+// The panel needs few SMs for long (161 us at n = 1728), the update all of them
+// (127 us): the next panel's columns are updated first, and its panel then runs
+// on a second stream beside the update of the rest.
 //  * gj_update_kernel: the rank-w update, 64 x 64 tiles.  A tile whose
 //    multipliers are all zero is left alone: the bottom operator couples
 //    neighbouring planes only, so most of the rows below a panel are.
 // The elimination of one column per launch that this replaces read and wrote
 // the whole n x 2n array [M | I] for each of the n columns: n = 1728 (8x8x9
-// nodes) took 55 ms; now 16.3 ms, of which the panels are 8.7 and the updates
+// nodes) took 55 ms, now 13 ms; the panels alone take 8.8 and the updates
 // 6.8 (5.4 at the FP64 pipe's rate without the empty tiles).
 #include <algorithm>
 
@@ -58,6 +61,17 @@ __device__ __forceinline__ long long magnitude(double v) { return __double_as_lo
 __device__ __forceinline__ bool no_pivot(long long m) { return m <= 0 || m >= 0x7ff0000000000000ll; }
 __device__ __forceinline__ bool better(long long m, int i, long long than, int at) {
     return m > than || (m == than && (unsigned)i < (unsigned)at);
+}
+
+// 1/v to within an ulp or two, by two Newton steps from FP32's reciprocal: five
+// FP64 instructions on the elimination's critical path, where the division is
+// twice that.  Values out of FP32's range take the division.
+__device__ __forceinline__ double reciprocal(double v) {
+    const unsigned e = (unsigned)(__double_as_longlong(v) >> 52) & 0x7ff;
+    if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / v;
+    double y = (double)(1.0f / (float)v);
+    y = fma_rn(fma_rn(-v, y, 1.0), y, y);
+    return fma_rn(fma_rn(-v, y, 1.0), y, y);
 }
 
 // What a CTA sends for a column: its pivot candidate (the largest magnitude
@@ -128,7 +142,7 @@ __global__ void __launch_bounds__(kPanelThreads)
             if (better(offers[b][d].mag, offers[b][d].index, best, at))
                 best = offers[b][d].mag, at = offers[b][d].index, from = d;
         if (tid < w) {
-            const double inv = 1.0 / offers[b][from].row[k];
+            const double inv = reciprocal(offers[b][from].row[k]);
             prow[tid] = tid == k ? inv : offers[b][from].row[tid] * inv;
             // rows c and the pivot's change places
             if (at >= r0 && at < r0 + mine) s[tid * rows + at - r0] = own[b][tid];
@@ -198,12 +212,14 @@ __global__ void __launch_bounds__(64)
 
 constexpr int kTile = 64;
 
-// A(:, q) += panel(:, .) rows(., q) for every column q outside the panel.
+// A(:, q) += panel(:, .) rows(., q) for the columns q of [q_lo, q_hi) that are
+// not in [skip_lo, skip_hi).
 template <int W>
 __global__ void __launch_bounds__(256)
-    gj_update_kernel(double *__restrict__ a, int n, int c0, int w, const double *__restrict__ rows) {
+    gj_update_kernel(double *__restrict__ a, int n, int c0, int w, int q_lo, int q_hi, int skip_lo, int skip_hi,
+                     const double *__restrict__ rows) {
     __shared__ double m[W][kTile + 1], v[W][kTile];
-    const int tid = threadIdx.x, i0 = blockIdx.y * kTile, q0 = blockIdx.x * kTile;
+    const int tid = threadIdx.x, i0 = blockIdx.y * kTile, q0 = q_lo + blockIdx.x * kTile;
     int some = 0, filled = 0;
     for (int t = tid; t < kTile * W; t += 256) {
         const int i = t / W, e = t % W;
@@ -211,7 +227,7 @@ __global__ void __launch_bounds__(256)
         m[e][i] = f;
         some |= magnitude(f) != 0;
         const int q = t % kTile, k = t / kTile;
-        const bool in = q0 + q < n && k < w && !(q0 + q >= c0 && q0 + q < c0 + w);
+        const bool in = q0 + q < q_hi && k < w && !(q0 + q >= skip_lo && q0 + q < skip_hi);
         const double g = in ? rows[(size_t)k * n + q0 + q] : 0.0;
         v[k][q] = g;
         filled |= magnitude(g) != 0;
@@ -242,7 +258,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
         for (int z = 0; z < 4; z++) {
             const int i = i0 + ty + 16 * u, q = q0 + tx + 16 * z;
-            if (i < n && q < n && !(q >= c0 && q < c0 + w)) a[(size_t)i * n + q] += acc[u][z];
+            if (i < n && q < q_hi && !(q >= skip_lo && q < skip_hi)) a[(size_t)i * n + q] += acc[u][z];
         }
 }
 
@@ -437,7 +453,7 @@ int panel_ctas(int n) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(16);
     cfg.blockDim = dim3(kPanelThreads);
-    cfg.dynamicSmemBytes = (n + 15) / 16 * W * sizeof(double);
+    cfg.dynamicSmemBytes = kPanelSmem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 16;
@@ -453,25 +469,63 @@ int panel_ctas(int n) {
 }
 
 template <int W>
+void launch_panel(double *a, int n, int c0, int ctas, int *pivots, int *bad, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(kPanelThreads);
+    // all of an SM's shared memory, so that no block of an update shares its FP64 pipe
+    cfg.dynamicSmemBytes = kPanelSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, gj_panel_kernel<W>, a, n, c0, std::min(W, n - c0), ctas, (n + ctas - 1) / ctas, pivots, bad);
+}
+
+// A second stream, of the highest priority, and the events that order it.
+struct SideStream {
+    cudaStream_t st = nullptr;
+    cudaEvent_t ready = nullptr, done = nullptr;
+    SideStream() {
+        int low = 0, high = 0;
+        cudaDeviceGetStreamPriorityRange(&low, &high);
+        if (cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, high) != cudaSuccess) st = nullptr;
+        if (cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) != cudaSuccess) ready = nullptr;
+        if (cudaEventCreateWithFlags(&done, cudaEventDisableTiming) != cudaSuccess) done = nullptr;
+    }
+    bool ok() const { return st && ready && done; }
+    ~SideStream() {   // all three end when the work that uses them has
+        if (ready) cudaEventDestroy(ready);
+        if (done) cudaEventDestroy(done);
+        if (st) cudaStreamDestroy(st);
+    }
+};
+
+template <int W>
 void eliminate(double *a, int n, double *rows, int *pivots, int *bad, cudaStream_t st) {
-    const int ctas = panel_ctas<W>(n), per = (n + ctas - 1) / ctas;
-    const int tiles = (n + kTile - 1) / kTile;
+    const int ctas = panel_ctas<W>(n), tiles = (n + kTile - 1) / kTile;
+    SideStream side;
+    launch_panel<W>(a, n, 0, ctas, pivots, bad, st);
     for (int c0 = 0; c0 < n; c0 += W) {
-        const int w = std::min(W, n - c0);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(ctas);
-        cfg.blockDim = dim3(kPanelThreads);
-        cfg.dynamicSmemBytes = per * W * sizeof(double);
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = ctas;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, gj_panel_kernel<W>, a, n, c0, w, ctas, per, pivots, bad);
+        const int w = std::min(W, n - c0), c1 = c0 + w, c2 = std::min(n, c1 + W);
         gj_rows_kernel<W><<<(n + 63) / 64, 64, 0, st>>>(a, n, c0, w, pivots, rows);
-        gj_update_kernel<W><<<dim3(tiles, tiles), 256, 0, st>>>(a, n, c0, w, rows);
+        if (c1 < n) {
+            gj_update_kernel<W><<<dim3(1, tiles), 256, 0, st>>>(a, n, c0, w, c1, c2, c0, c1, rows);
+            if (side.ok()) {
+                cudaEventRecord(side.ready, st);
+                cudaStreamWaitEvent(side.st, side.ready, 0);
+                launch_panel<W>(a, n, c1, ctas, pivots, bad, side.st);
+                cudaEventRecord(side.done, side.st);
+            }
+        }
+        gj_update_kernel<W><<<dim3(tiles, tiles), 256, 0, st>>>(a, n, c0, w, 0, n, c0, c2, rows);
+        if (c1 < n) {
+            if (side.ok()) cudaStreamWaitEvent(st, side.done, 0);
+            else launch_panel<W>(a, n, c1, ctas, pivots, bad, st);
+        }
     }
 }
 
