@@ -238,6 +238,15 @@ __device__ __forceinline__ T dot3(T a0, T b0, T a1, T b1, T a2, T b2) {
     return fma_rn(a2, b2, fma_rn(a1, b1, mul_rn(a0, b0)));
 }
 
+// FP32 to FP64 by the bits where the value is a normal number: a conversion
+// takes the FP64 pipe as long as a product.
+__device__ __forceinline__ double widen(float v) {
+    const unsigned u = __float_as_uint(v), e = u >> 23 & 255;
+    if (e - 1 > 253) return (double)v;
+    return __hiloint2double((int)((u & 0x80000000u) | ((u & 0x7fffffffu) >> 3) + 0x38000000u), (int)(u << 29));
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
 template <typename T>
 __device__ inline void matvec_sub(const T *a, const T *v, T *acc) {
     acc[0] -= dot3(a[0], v[0], a[1], v[1], a[2], v[2]);

@@ -46,11 +46,26 @@ __global__ void slice_kernel(Geom g, const double *__restrict__ f, int k, int qu
 
 constexpr int kG = 2;   // ghost layers of the simulation grid
 
+// float(sqrt(q)) with the square root correctly rounded in FP64 first.  One
+// Newton step from FP32's reciprocal root gives the root to 2^-42; the float
+// it rounds to is the same unless it lies that near the middle between two
+// floats, where the root is taken exactly, as it is out of FP32's range.  Four
+// FP64 instructions for thirteen.
+__device__ __forceinline__ float root(double q) {
+    const unsigned e = (unsigned)(__double_as_longlong(q) >> 52);   // the sign too: negative is out of range
+    if (e - (1023 - 100) > 200) return __double2float_rn(__dsqrt_rn(q));
+    const float yf = rsqrtf((float)q);
+    const double s0 = q * widen(yf), s = __fma_rn(__fma_rn(-s0, s0, q), widen(0.5f * yf), s0);
+    const int past = (int)(__double_as_longlong(s) & 0x1fffffff) - 0x10000000;   // from the middle, in units of 2^-52
+    if (abs(past) < 1 << 12) return __double2float_rn(__dsqrt_rn(q));
+    return __double2float_rn(s);
+}
+
 // The fields run along x and the output along z, so a block turns a tile of 32
 // x 32 values of one y over in shared memory: written straight from the
 // threads that read it, every value of one of the two sides took a sector of
 // its own (192^3 points: a velocity 68 us, the deviatoric stress 688 us, now
-// 29 and 349 us).  The deviatoric stress is bound by the FP64 pipe: its
+// 29 and 323 us).  The deviatoric stress is bound by the FP64 pipe: its
 // sums and products are fused multiply-adds by 1 and onto -0 where that saves
 // the pipe three cycles in nineteen, with constants the compiler cannot see.
 constexpr int kTile = 32;
@@ -68,6 +83,7 @@ __global__ void __launch_bounds__(256) cube_kernel(stz_cube_fields f, int nx, in
             if (xx >= nx || zz >= zsize) continue;
             const long p = (xx + kG) + sy * (yy + kG) + sz * (zz + kG);
             double v = 0;
+            float root_of = 0.0f;   // mode 10
             switch (mode) {   // Field::fval (src/field.hh:157-177)
                 case 0: v = f.u[p]; break;
                 case 1: v = f.v[p]; break;
@@ -90,7 +106,7 @@ __global__ void __launch_bounds__(256) cube_kernel(stz_cube_fields f, int nx, in
                         const double s12 = f.s12[p], s13 = f.s13[p], s23 = f.s23[p];
                         // half of an exact sum's double: one rounding, of the addition
                         const double q = __fma_rn(0.5, sq3(t11, t22, t33), ml(s12, s12));
-                        v = __dsqrt_rn(ad(ad(q, ml(s13, s13)), ml(s23, s23)));
+                        root_of = root(ad(ad(q, ml(s13, s13)), ml(s23, s23)));
                     }
                     break;
                 }
@@ -100,7 +116,7 @@ __global__ void __launch_bounds__(256) cube_kernel(stz_cube_fields f, int nx, in
                 case 14: v = f.xi_y[p]; break;
                 default: v = f.xi_z[p]; break;
             }
-            tile[zt][threadIdx.x] = __double2float_rn(v);
+            tile[zt][threadIdx.x] = mode == 10 ? root_of : __double2float_rn(v);
         }
         __syncthreads();
         const int zz = z0 + threadIdx.x;

@@ -219,15 +219,6 @@ __global__ void scale_kernel(double *__restrict__ v, double s, size_t n) {
     for (; t < n; t += (size_t)gridDim.x * blockDim.x) v[t] *= s;
 }
 
-// FP32 to FP64 by the bits where the value is a normal number: a conversion
-// takes the FP64 pipe as long as a product.
-__device__ __forceinline__ double widen(float v) {
-    const unsigned u = __float_as_uint(v), e = u >> 23 & 255;
-    if (e - 1 > 253) return (double)v;
-    return __hiloint2double((int)((u & 0x80000000u) | ((u & 0x7fffffffu) >> 3) + 0x38000000u), (int)(u << 29));
-}
-__device__ __forceinline__ double widen(double v) { return v; }
-
 // x = Ainv r, a warp per row (Ainv row-major, lanes stride the columns), a row
 // per scheduler and block.  r is gathered and widened once per block: a look-up
 // and an FP64 conversion per matrix entry took the 1728-row product of an FP32
