@@ -7,18 +7,19 @@
 // and after all of them the array is the inverse of the row-permuted matrix.
 //
 // Three launches a panel:
-//  * gj_panel_kernel: one cluster of 16 CTAs (8 where 16 do not fit) holds the panel in shared memory,
-//    rows spread over the CTAs, and eliminates its columns one by one.  Per
-//    column every CTA sends its pivot candidate, with the candidate's whole
-//    row, to the others, so one cluster barrier a column is enough.
+//  * gj_panel_kernel: one cluster of 16 CTAs (8 where 16 do not fit) holds the
+//    panel in shared memory, rows spread over the CTAs, and eliminates its
+//    columns one by one.  Per column every CTA sends its pivot candidate, with
+//    the candidate's whole row, to the others, so one cluster barrier a column
+//    is enough.
 //  * gj_rows_kernel: the row swaps on the other columns; the pivot rows'
 //    values go to a w x n scratch.
-// The panel needs few SMs for long (161 us at n = 1728), the update all of them
-// (127 us): the next panel's columns are updated first, and its panel then runs
-// on a second stream beside the update of the rest.
 //  * gj_update_kernel: the rank-w update, 64 x 64 tiles.  A tile whose
 //    multipliers are all zero is left alone: the bottom operator couples
 //    neighbouring planes only, so most of the rows below a panel are.
+// The panel needs few SMs for long (161 us at n = 1728), the update all of them
+// (127 us): the next panel's columns are updated first, and its panel then runs
+// on a second stream beside the update of the rest.
 // The elimination of one column per launch that this replaces read and wrote
 // the whole n x 2n array [M | I] for each of the n columns: n = 1728 (8x8x9
 // nodes) took 55 ms, now 13 ms; the panels alone take 8.8 and the updates
@@ -295,15 +296,20 @@ __global__ void gj_gather_kernel(const double *__restrict__ a, int n, const int 
 // shared memory by the same elimination as above.  On the host, one system
 // after the other, 64 systems of order 27 took 11.6 ms; here 134 us.
 constexpr int kFourierThreads = 256;
-constexpr int kFourierOrder = 112;   // two arrays of order^2 doubles in shared memory
+constexpr int kFourierOrder = 104;   // two arrays of order^2 doubles in shared memory
 
+// work: null, or 2 bs^2 doubles per CTA for systems beyond shared memory.
 __global__ void __launch_bounds__(kFourierThreads)
-    fourier_inverse_kernel(Geom g, PlaneOp<double> op, double2 *__restrict__ out, int *bad) {
+    fourier_inverse_kernel(Geom g, PlaneOp<double> op, double2 *__restrict__ out, double *work, int *bad) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int bs = 3 * g.o, tid = threadIdx.x, kx = blockIdx.x % g.m, ky = blockIdx.x / g.m;
-    double *re = reinterpret_cast<double *>(smem), *im = re + bs * bs;
-    __shared__ double2 wx[3], wy[3], prow[kFourierOrder], col[kFourierOrder];
-    __shared__ int piv, order[kFourierOrder], pivots[kFourierOrder];
+    double2 *prow = reinterpret_cast<double2 *>(smem), *col = prow + bs;
+    int *order = reinterpret_cast<int *>(col + bs), *pivots = order + bs;
+    double *re = work ? work + 2 * (size_t)blockIdx.x * bs * bs
+                      : reinterpret_cast<double *>(smem + (size_t)bs * (2 * sizeof(double2) + 2 * sizeof(int)));
+    double *im = re + bs * bs;
+    __shared__ double2 wx[3], wy[3];
+    __shared__ int piv;
     if (tid < 6) {   // e^{i t d}
         const int d = tid % 3 - 1;
         double sn, cs;
@@ -350,12 +356,12 @@ __global__ void __launch_bounds__(kFourierThreads)
         // swap rows c and piv; the pivot row over the pivot, and column c
         const int p = piv;
         const double pr = re[p * bs + c], pi = im[p * bs + c];
-        if (tid < bs) {
+        for (int e = tid; e < bs; e += kFourierThreads) {
             const double s2 = 1.0 / (pr * pr + pi * pi), ir = pr * s2, ii = -pi * s2;
-            const double ur = re[p * bs + tid], ui = im[p * bs + tid];
-            prow[tid] = tid == c ? make_double2(ir, ii) : make_double2(ur * ir - ui * ii, ur * ii + ui * ir);
-            const int r = tid == p ? c : tid;   // the row whose values are at tid after the swap
-            col[tid] = make_double2(re[r * bs + c], im[r * bs + c]);
+            const double ur = re[p * bs + e], ui = im[p * bs + e];
+            prow[e] = e == c ? make_double2(ir, ii) : make_double2(ur * ir - ui * ii, ur * ii + ui * ir);
+            const int r = e == p ? c : e;   // the row whose values are at e after the swap
+            col[e] = make_double2(re[r * bs + c], im[r * bs + c]);
         }
         __syncthreads();
         for (int t = tid; t < bs * bs; t += kFourierThreads) {
@@ -531,17 +537,22 @@ void eliminate(double *a, int n, double *rows, int *pivots, int *bad, cudaStream
 
 }  // namespace
 
-// False where the blocks are too many for scratch (n x n doubles) or shared memory.
+// False where the blocks would not fit the scratch (n x n doubles): one or two
+// columns, for which the plain inverse is as good.
 bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, double *inv, double *scratch, int *bad,
                             cudaStream_t st) {
     const int bs = 3 * g.o, cols = g.m * g.n, n = bs * cols;
-    if (!g.xp || !g.yp || cols < 3 || cols > 2048 || bs > kFourierOrder) return false;
-    const int smem = 2 * bs * bs * (int)sizeof(double);
+    if (!g.xp || !g.yp || cols < 3) return false;
+    // systems beyond shared memory work in the inverse's place, which is written last
+    const bool fits = bs <= kFourierOrder;
+    const int smem = bs * (int)(2 * sizeof(double2) + 2 * sizeof(int)) + (fits ? 2 * bs * bs * (int)sizeof(double) : 0);
+    const int phases = cols * (int)sizeof(double2);   // 64 KB at the 4096 nodes a direct bottom may have
     cudaFuncSetAttribute(fourier_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(fourier_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, phases);
     double2 *G = reinterpret_cast<double2 *>(scratch);
     double *B = scratch + 2 * (size_t)cols * bs * bs;
-    fourier_inverse_kernel<<<cols, kFourierThreads, smem, st>>>(g, op, G, bad);
-    fourier_blocks_kernel<<<dim3((bs * bs + 127) / 128, cols), 128, cols * sizeof(double2), st>>>(g.m, g.n, bs, G, B);
+    fourier_inverse_kernel<<<cols, kFourierThreads, smem, st>>>(g, op, G, fits ? nullptr : inv, bad);
+    fourier_blocks_kernel<<<dim3((bs * bs + 127) / 128, cols), 128, phases, st>>>(g.m, g.n, bs, G, B);
     fourier_expand_kernel<<<dim3((n + 255) / 256, n), 256, 0, st>>>(g, B, inv);
     return true;
 }

@@ -51,3 +51,31 @@ def test_bottom_inverse(dims, per):
     # the forward error of a pivoted elimination of order n: n eps cond(M), with room for its growth
     ref = np.linalg.solve(M, b.reshape(-1))
     assert np.linalg.norm(x - ref) <= 64 * len(M) * 2.0 ** -53 * np.linalg.cond(M) * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("dims,per", [((8, 8, 66), (True, True, False)), ((8, 8, 68), (True, True, False)),
+                                      ((8, 8, 200), (True, True, False)), ((92, 92, 2), (True, True, True))])
+def test_fourier_inverse_of_tall_columns_and_many(dims, per, monkeypatch):
+    """Columns of 34 and 35 planes (systems of order 102, the last in shared
+    memory, and 105, the first beyond it), of 101 planes (order 303: more
+    rows than a CTA has threads), and 2116 columns of one plane: a V-cycle with
+    the Fourier inverse against one with the plain inverse.  The shift bounds the bottom's condition by 100, so
+    the two inverses differ by at most 64 n eps 100 of the solution."""
+    import stzpp_gb300 as sg
+    m, n, o = dims
+    st, fix = sg.elastic_stencil(1.0, 2.0, *P.grid_spacing(m, n, o, per, h=1.0 / 8))
+    st = np.array(st).reshape(27, 3, 3)
+    st[13] += np.diag(np.diag(st[13]))
+    b = np.random.default_rng(2).standard_normal((m * n * o, 3))
+    x = []
+    for fourier in ("0", "1"):
+        monkeypatch.setenv("STZ_MG_BOTTOM_FOURIER", fourier)
+        with sg.Multigrid(dims, per, precision="fp64", max_coarse=m * n * o // 3, bottom="direct") as mg:
+            mg.setup_matrices(stencil=st.reshape(27, 9), fix=fix)
+            mg.setup_fields(r=b)
+            mg.v_cycle()
+            assert mg.nlevels == 2
+            x.append(mg.get_x())
+    assert np.isfinite(x[0]).all() and np.abs(x[0]).max() > 0
+    order = 3 * m * n * o // 4
+    assert np.linalg.norm(x[1] - x[0]) <= 64 * order * 2.0 ** -53 * 100 * np.linalg.norm(x[0])
