@@ -115,6 +115,7 @@ struct AdvConst {
     Divisor c0, sy, mu, bath, tau0, syc0;   // syc0: sy*c0 (calc_chi_F)
     double mu2;             // 2*mu
     double oe;              // omega*eps0
+    double elastic;         // 0./2./mu: the new ad_Dpl of a cell below the yield stress over its sbar
 };
 
 // Cell t of the interior, x fastest.  Threads take consecutive cells across
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(kThreads)
             above = sbar0 > P.sy;
             if (!above) {
                 adapt_out[p] = 0.0;
-                adnew[p] = ml(0.0, sbar0);
+                adnew[p] = ml(C.elastic, sbar0);
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, above);
@@ -412,6 +413,7 @@ extern "C" int stz_mg_advection_step(const stz_adv_params *P, const stz_adv_fiel
     C.syc0 = divisor(P->sy * P->c0);
     C.mu2 = 2.0 * P->mu;
     C.oe = P->omega * P->eps0;
+    C.elastic = 0.0 / P->mu;
     // work: adaptive terms, new ad_Dpl, then flags {a cell yielded, a cell hit kMaxSubsteps}
     double *adapt = f->work, *adnew = f->work + g.npts, *flag = f->work + 2 * g.npts;
     if (cudaMemsetAsync(flag, 0, 2 * sizeof(double), st) != cudaSuccess) return STZ_MG_ERR_CUDA;
