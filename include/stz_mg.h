@@ -229,7 +229,7 @@ int stz_mg_time_kernel(stz_mg_handle h, int kernel, int level, int reps, double 
 /* Measurement hook (no counterpart in the reference): how the solver sweeps
  * a level in its precision -- STZ_MG_SWEEP_COLOUR (eight colour launches per
  * sweep), _TILE (two-buffer tiles), _BAND (full-width bands staged by TMA),
- * _PHASE (a block per plane) -- and the kernel launches of one sweep. */
+ * _PHASE (a block or cluster per plane) -- and the kernel launches of one sweep. */
 enum { STZ_MG_SWEEP_COLOUR = 0, STZ_MG_SWEEP_TILE = 1, STZ_MG_SWEEP_BAND = 2, STZ_MG_SWEEP_PHASE = 3 };
 int stz_mg_sweep_kind(stz_mg_handle h, int level, int *kind, int *launches_per_sweep);
 

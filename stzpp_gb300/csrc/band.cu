@@ -1,8 +1,8 @@
-// Band Gauss-Seidel sweep of the levels periodic in x and y -- the fine
-// level's shared elasticity stencil and the plane-invariant coarse operators
-// below it -- two launches per sweep, every CTA staging its planes with the
-// tensor-memory-access (TMA) engine; and the band residual of the
-// plane-invariant levels from the same staging.
+// Band Gauss-Seidel sweep of the levels periodic in x and y of up to 256 nodes
+// a row -- shared stencils (elasticity or full blocks), the plane-invariant
+// coarse operators below them, and FP32 Lame levels -- two launches per sweep,
+// every CTA staging its planes with the tensor-memory-access (TMA) engine; and
+// the band residual of the plane-invariant levels from the same staging.
 //
 // Replaces, on those levels, the eight colour launches of smooth.cu
 // (region::gauss_seidel, region.cc:1557-1762,
@@ -27,8 +27,8 @@
 //  * the planes above and below are old (x_in, even launch) or new (x_out,
 //    odd launch) values, as in the colour order.
 //
-// Each node update has the arithmetic of const_row (ops.cuh) in the same
-// order, so the sweep is bit-identical to the eight colour launches.  Every
+// Each node update has the arithmetic of const_row, plane_row_coef or lame_row
+// (ops.cuh) in the same order, so the sweep is bit-identical to the eight colour launches.  Every
 // wait is an mbarrier wait with a time limit; a CTA whose copies do not
 // arrive in time records the fact (band_take_error) and returns.
 #include <cuda.h>
@@ -1176,9 +1176,10 @@ bool launch_band_op(const LevelOp<T> &op, const Geom &g, const T *r, const T *xi
 }  // namespace
 
 // Where the band sweep runs: a shared stencil, a plane-invariant coarse
-// operator or (FP32) per-node Lame coefficients, a level periodic in x and y, rows of up to 256 nodes whose colours
-// are whole 16-byte units (the tensor maps' strides), whole bands of 8 rows
-// (at least two), an even z extent if z is periodic.  FP32 levels by default;
+// operator or (FP32) per-node Lame coefficients, a level periodic in x and y,
+// rows of up to 256 nodes whose colours are whole 16-byte units (the tensor
+// maps' strides), whole bands of 8 rows (at least two), an even z extent if z
+// is periodic.  FP32 levels by default;
 // STZ_MG_BAND=0 turns it off, STZ_MG_BAND=1 uses it in FP64 too.
 template <typename T>
 bool gs_band_applies(const LevelOp<T> &op, const Geom &g) {

@@ -313,8 +313,9 @@ void launch_gs_colour(const LevelOp<T> &op, const Geom &g, int q, const T *r, T 
 }
 
 // Large planes: one launch per colour keeps millions of threads in flight;
-// the plane-phase kernels (one block per plane) pay off where a colour of a
-// plane is at most two nodes per thread, i.e. where launch latency dominates.
+// the plane-phase kernels (one block per plane; shared stencils and Lame levels
+// that the bands do not take) pay off where a colour of a plane is at most two
+// nodes per thread, i.e. where launch latency dominates.
 // (An odd periodic z would put both parities of a colour on one plane.)
 static bool odd_periodic_z(const Geom &g) { return g.zp && (g.o & 1) && g.o > 1; }
 
