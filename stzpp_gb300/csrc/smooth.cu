@@ -321,8 +321,11 @@ static bool odd_periodic_z(const Geom &g) { return g.zp && (g.o & 1) && g.o > 1;
 
 template <typename T>
 static bool large_planes(const LevelOp<T> &op, const Geom &g) {
-    // dense.cu and plane.cu take planes of any size
-    if (op.kind == OP_DENSE || (op.kind == OP_PLANE && sizeof(T) == 8)) return odd_periodic_z(g);
+    // dense.cu and plane.cu take planes of any size.  They read the planes above
+    // and below ahead of a colour's end, so those must not be the plane itself:
+    // a single periodic plane takes the colour launches.
+    if ((op.kind == OP_DENSE || op.kind == OP_PLANE) && g.zp && (g.o & 1)) return true;
+    if (op.kind == OP_DENSE || (op.kind == OP_PLANE && sizeof(T) == 8)) return false;
     const int phase_max = sizeof(T) == 8 ? 256 : 2 * kPhaseThreads;   // FP64 needs every SM's FP64 units
     return odd_periodic_z(g) || g.M2 * g.N2 > phase_max;
 }

@@ -69,3 +69,27 @@ def test_dense_residual(dims, per):
     assert (np.abs(got.reshape(ref.shape) - ref) <= 2 * 84 * 2.0 ** -53 * size).all()
     total = float((got ** 2).sum())
     assert abs(sq - total) <= 1e-13 * total
+
+
+@pytest.mark.parametrize("dims", [(12, 10, 1), (34, 18, 1)])
+def test_single_periodic_plane(dims):
+    """The planes above and below a single periodic plane are itself: a colour
+    pass reads what the one before wrote there.  Against the same order of
+    updates in numpy."""
+    per = (True, True, True)
+    mg, A = handle(dims, per)
+    x, r = fields(dims, 9)
+    mg.set_x(x)
+    mg.set_rhs(r)
+    mg.gauss_seidel(0, 2)
+    m, n, o = dims
+    A = np.asarray(A).reshape(n, m, 27, 3, 3)
+    X, R = x.reshape(n, m, 3).copy(), r.reshape(n, m, 3)
+    for q in 2 * [(0, 0), (1, 0), (0, 1), (1, 1)]:
+        for j in range(q[1], n, 2):
+            for i in range(q[0], m, 2):
+                s = R[j, i] - sum(A[j, i, b] @ X[(j + b // 3 % 3 - 1) % n, (i + b % 3 - 1) % m]
+                                  for b in range(27) if b != 13)
+                X[j, i] = np.linalg.solve(A[j, i, 13], s)
+    assert np.abs(mg.get_x().reshape(X.shape) - X).max() <= 1e-12 * np.abs(X).max()
+    assert mg.sweep_kind(0) == ("colour", 8)

@@ -69,3 +69,30 @@ def test_plane_residual(dims, elastic, level):
         size += np.einsum("kjirc,kjic->kjir", np.abs(A[..., b, :, :]), np.abs(nb))
     # 81 products and 82 additions, each rounded once on either side
     assert (np.abs(got.reshape(ref.shape) - ref) <= 2 * 84 * 2.0 ** -53 * size).all()
+
+
+def test_single_periodic_plane():
+    """A level of one periodic plane, whose planes above and below are itself,
+    sweeps by the colour launches."""
+    import stzpp_gb300 as sg
+    dims, per = (24, 20, 2), (True, True, True)
+    st, fix = sg.elastic_stencil(1.0, 2.0, *P.grid_spacing(*dims, per, h=1.0 / 8))
+    st = np.array(st).reshape(27, 3, 3)
+    st[13] += np.diag(np.diag(st[13]))
+    mg = sg.Multigrid(dims, per, precision="fp64", max_coarse=200, bottom="gs")
+    mg.setup_matrices(st.reshape(27, 9), fix)
+    assert tuple(mg.level_dims(1)) == (12, 10, 1)
+    rng = np.random.default_rng(7)
+    x, r = rng.standard_normal((120, 3)), rng.standard_normal((120, 3))
+    out = []
+    for whole in (True, False):
+        mg.level_set_field(1, "x", x)
+        mg.level_set_field(1, "r", r)
+        if whole:
+            mg.gauss_seidel(1, 2)
+        else:
+            for _ in range(2):
+                mg.gauss_seidel_colours(1, 0, 8)
+        out.append(mg.level_get_field(1, "x"))
+    assert np.array_equal(out[0], out[1])
+    assert mg.sweep_kind(1) == ("colour", 8)
