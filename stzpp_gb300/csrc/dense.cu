@@ -24,11 +24,15 @@
 // the colour before is loaded ahead of the barrier: the coefficients, and x of
 // the planes above and below.
 //
+// On levels too small to fill the SMs a colour's chain is left: 21 FP64
+// multiply-adds in a row, the sum, the store, the barrier and the loads, 3.4 us
+// (all sweeps of 7x6x5 in one launch: 27.5 -> 26.9 us each, not kept).
+//
 // One sweep on GB300, before (one block a plane on planes of up to 64x64,
 // else eight colour launches, a thread a node) and now:
 //   64x64x65  FP32  310 -> 69 us     16x16x17  FP32   54 -> 14 us
 //   49x41x33  FP64  328 -> 148 us    32x48x26  FP64  245 -> 66 us
-//   7x6x5     FP64  118 -> 31 us
+//   7x6x5     FP64  118 -> 28 us
 // and the residual of 49x41x33 in FP64 72 -> 59 us, of 16x16x17 in FP32 23 -> 3 us.
 #include <algorithm>
 
