@@ -489,7 +489,7 @@ void build_bottom(stz_mg_handle h) {
     // (STZ_MG_BOTTOM_FOURIER=0 turns that off)
     const char *fe = std::getenv("STZ_MG_BOTTOM_FOURIER");
     h->bottom_fourier = !(fe && std::atoi(fe) == 0) && h->op64[lb].kind == OP_PLANE &&
-                        launch_fourier_inverse(h->op64[lb].pop, g, h->ainv_t, h->bot_a, h->dflag, h->st);
+                        launch_fourier_inverse(h->op64[lb].pop, g, h->S[lb], h->ainv_t, h->bot_a, h->dflag, h->st);
     if (!h->bottom_fourier) {
         const double *rows = h->op64[lb].dop.coef;
         if (h->op64[lb].kind != OP_DENSE) {

@@ -424,6 +424,24 @@ __global__ void fourier_expand_kernel(Geom g, const double *__restrict__ B, doub
     inv[(size_t)r * nr + q] = B[((size_t)(di + g.m * dj) * bs + 3 * k + r % 3) * bs + 3 * k2 + q % 3];
 }
 
+__device__ __forceinline__ bool beyond_one_node(const Geom &g, const int *S, int s) {
+    bool far = false;
+#pragma unroll
+    for (int e = 0; e < 6; e++) {
+        const int v = S[(size_t)e * g.npad + s];
+        far |= e & 1 ? v > 2 : v < -1;
+    }
+    return far;
+}
+
+// bad[1] is set when a node's box reaches beyond one node.
+__global__ void box_check_kernel(Geom g, const int *__restrict__ S, int *bad) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= g.m * g.n * g.o) return;
+    const int s = slot(g, p % g.m, p / g.m % g.n, p / (g.m * g.n));
+    if (beyond_one_node(g, S, s)) atomicExch(bad + 1, 1);
+}
+
 // M (n x n, natural node order, 3 rows per node) from grouped rows and box
 // bounds: the blocks of a node's box, added where wraps make two of them
 // meet.  bad[1] is set when a box reaches beyond one node.
@@ -539,8 +557,8 @@ void eliminate(double *a, int n, double *rows, int *pivots, int *bad, cudaStream
 
 // False where the blocks would not fit the scratch (n x n doubles): one or two
 // columns, for which the plain inverse is as good.
-bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, double *inv, double *scratch, int *bad,
-                            cudaStream_t st) {
+bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, const int *S, double *inv, double *scratch,
+                            int *bad, cudaStream_t st) {
     const int bs = 3 * g.o, cols = g.m * g.n, n = bs * cols;
     if (!g.xp || !g.yp || cols < 3) return false;
     // systems beyond shared memory work in the inverse's place, which is written last
@@ -551,6 +569,7 @@ bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, double *in
     cudaFuncSetAttribute(fourier_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, phases);
     double2 *G = reinterpret_cast<double2 *>(scratch);
     double *B = scratch + 2 * (size_t)cols * bs * bs;
+    box_check_kernel<<<(g.m * g.n * g.o + 127) / 128, 128, 0, st>>>(g, S, bad);
     fourier_inverse_kernel<<<cols, kFourierThreads, smem, st>>>(g, op, G, fits ? nullptr : inv, bad);
     fourier_blocks_kernel<<<dim3((bs * bs + 127) / 128, cols), 128, phases, st>>>(g.m, g.n, bs, G, B);
     fourier_expand_kernel<<<dim3((n + 255) / 256, n), 256, 0, st>>>(g, B, inv);

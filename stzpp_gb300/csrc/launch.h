@@ -166,7 +166,7 @@ void launch_bottom_matrix(const Geom &g, const double *coef, const int *S, doubl
 // the same inverse of a plane-invariant bottom level periodic in x and y from
 // its Fourier blocks (scratch: as many doubles as the inverse); false where
 // that does not apply
-bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, double *inv, double *scratch, int *bad,
+bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, const int *S, double *inv, double *scratch, int *bad,
                             cudaStream_t st);
 void launch_gauss_jordan(double *a, int n, double *inv, int *pivots, double *rows, int *bad, cudaStream_t st);
 

@@ -79,3 +79,18 @@ def test_fourier_inverse_of_tall_columns_and_many(dims, per, monkeypatch):
     assert np.isfinite(x[0]).all() and np.abs(x[0]).max() > 0
     order = 3 * m * n * o // 4
     assert np.linalg.norm(x[1] - x[0]) <= 64 * order * 2.0 ** -53 * 100 * np.linalg.norm(x[0])
+
+
+@pytest.mark.parametrize("fourier", ["0", "1"])
+def test_box_beyond_one_node_is_refused(fourier, monkeypatch):
+    """A level coarsened from a single periodic plane has boxes of more than
+    one node: no direct bottom, whichever inverse would run."""
+    import stzpp_gb300 as sg
+    dims, per = (16, 16, 2), (True, True, True)
+    st, fix = sg.elastic_stencil(1.0, 2.0, *P.grid_spacing(*dims, per, h=1.0 / 16))
+    st = np.array(st).reshape(27, 3, 3)
+    st[13] += np.diag(np.diag(st[13]))
+    monkeypatch.setenv("STZ_MG_BOTTOM_FOURIER", fourier)
+    with sg.Multigrid(dims, per, precision="fp64", max_coarse=20, bottom="direct") as mg:
+        with pytest.raises(sg.StzMgError, match="beyond one node"):
+            mg.setup_matrices(stencil=st.reshape(27, 9), fix=fix)
