@@ -10,8 +10,11 @@
 // plane's row lies in shared memory, and a warp goes down the blocks in the
 // order of plane_row_coef (ops.cuh), each entry a fused multiply-add, so that
 // the results are those of the colour launches bit for bit.  On planes with
-// the elasticity structure (PlaneOp::structured) a lane skips what is zero in
-// its row: 1, 2 or 3 products for a face, edge or corner block instead of 3.
+// the elasticity structure a lane skips what is zero in its row: 1, 2 or 3
+// products for a face, edge or corner block instead of 3.  Those are the planes
+// whose other entries are zero (PlaneOp::structured), and all planes where the
+// other kernels of the level skip them too (PlaneOp::sparse: in FP32 up to 1e-9
+// of the plane's largest entry).
 //
 // The sweep is two launches, the even planes and then the odd ones; a cluster
 // of up to 8 CTAs runs the four colours of a plane (region::gauss_seidel,
@@ -140,7 +143,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2)
     const int groups = (plane + kNodes - 1) / kNodes, rounds = (groups + warps - 1) / warps;
     const size_t np = (size_t)g.npad;
     const LaneRow L(row);
-    const bool sparse = op.structured[2 * K + c];
+    const bool sparse = op.sparse || op.structured[2 * K + c];
     stage_row(op, 2 * K + c, cf);
     chain_wait();
     NbrOffsets nb;
