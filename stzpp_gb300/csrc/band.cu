@@ -227,7 +227,7 @@ __device__ __forceinline__ void stage_coef(const PlaneOp<T> &pop, int k, T *cfs,
 // elasticity operators), with the arithmetic of const_row<T, SPARSE, false> or
 // plane_row_coef<T, SPARSE, false>.
 template <typename T, int M2, int KIND, bool SPARSE, int A, int B, int NR>
-__device__ __forceinline__ void band_colour(const T *__restrict__ s, const int (&ib)[3], const LevelOp<T> &op,
+__device__ __forceinline__ void band_colour(const T *s, const int (&ib)[3], const LevelOp<T> &op,
                                             const T *cf, int nvalid, const T (&rr)[NR][3], T (&out)[NR][3]) {
     constexpr bool CONST = KIND == OP_CONST;
     constexpr int rowstep = woff<M2>(0, 0, 1, 0, 0);
@@ -420,7 +420,7 @@ __device__ __forceinline__ void band_issue(const BandArgs &args, const BandMaps 
 // A Dirichlet plate of the shared stencil: x = fix^-1 r, no neighbours.
 template <typename T, int M2, int NH, bool PAD>
 __device__ __forceinline__ void band_plate(const Geom &g, const ConstOp<T> &op, const BandItem &it, int c,
-                                           const T *__restrict__ r, T *__restrict__ xout) {
+                                           const T *r, T *xout) {
     const int tid = threadIdx.x, I = tid % M2, hh = tid / M2;
     if (PAD && I >= g.M2) return;
     const size_t np = (size_t)g.npad;
@@ -442,8 +442,7 @@ __device__ __forceinline__ void band_plate(const Geom &g, const ConstOp<T> &op, 
 // arrive (recorded; every thread returns false).
 template <typename T, int M2, int NH, int KIND, bool SPARSE, bool PAD>
 __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp<T> &op, const BandItem &it, T *s,
-                                             T *cfs, unsigned bar, unsigned phase, const T *__restrict__ r,
-                                             T *__restrict__ xout) {
+                                             T *cfs, unsigned bar, unsigned phase, const T *r, T *xout) {
     const Geom &g = args.g;
     const int tid = threadIdx.x, I = tid % M2, hh = tid / M2;
     const int c = args.c, K = it.K, J0 = it.J0, k = it.k;
@@ -462,8 +461,8 @@ __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp
         const size_t s0 = band_slot(g, 0, c, K, J, I), s1 = band_slot(g, 1, c, K, J, I);
 #pragma unroll
         for (int cc = 0; cc < 3; cc++) {
-            r0[u][cc] = __ldcs(r + s0 + cc * np);
-            r1[u][cc] = __ldcs(r + s1 + cc * np);
+            r0[u][cc] = load_once(r + s0 + cc * np);
+            r1[u][cc] = load_once(r + s1 + cc * np);
         }
     }
 #pragma unroll
@@ -472,8 +471,8 @@ __device__ __forceinline__ bool band_compute(const BandArgs &args, const LevelOp
         const size_t s2 = band_slot(g, 2, c, K, J0 + t0b + u, I), s3 = band_slot(g, 3, c, K, J0 + t0b + u, I);
 #pragma unroll
         for (int cc = 0; cc < 3; cc++) {
-            r2[u][cc] = __ldcs(r + s2 + cc * np);
-            r3[u][cc] = __ldcs(r + s3 + cc * np);
+            r2[u][cc] = load_once(r + s2 + cc * np);
+            r3[u][cc] = load_once(r + s3 + cc * np);
         }
     }
     const bool ok = mbar_wait(bar, phase, 200000000ull);   // 0.2 s: copies that never arrive
@@ -560,7 +559,7 @@ constexpr int kBandMinBlocks =
 template <typename T, int M2, int NH, int KIND, bool SPARSE, bool PAD>
 __global__ void __launch_bounds__(NH * M2, (kBandMinBlocks<T, M2, KIND>))
     gs_band_kernel(const BandArgs args, const __grid_constant__ LevelOp<T> op, const __grid_constant__ BandMaps in,
-                   const __grid_constant__ BandMaps out_maps, const T *__restrict__ r, T *__restrict__ xout) {
+                   const __grid_constant__ BandMaps out_maps, const T *r, T *xout) {
     extern __shared__ __align__(128) unsigned char band_smem[];
     __shared__ __align__(8) unsigned long long bar_store;
     __shared__ __align__(16) T cfs[KIND == OP_PLANE ? kCoefWords : 4];
@@ -666,8 +665,7 @@ constexpr int kLamePer = (kLameRows<M2, B> + NH - 1) / NH;
 template <int M2, int NH, int A, int B>
 struct LameRhs {
     float v[kLamePer<M2, NH, B>][3];
-    __device__ __forceinline__ LameRhs(const BandArgs &args, const BandItem &it, int I, int hh,
-                                       const float *__restrict__ r) {
+    __device__ __forceinline__ LameRhs(const BandArgs &args, const BandItem &it, int I, int hh, const float *r) {
         const Geom &g = args.g;
 #pragma unroll
         for (int u = 0; u < kLamePer<M2, NH, B>; u++) {
@@ -675,7 +673,7 @@ struct LameRhs {
             if (I >= g.M2 || t >= kLameRows<M2, B>) break;
             const size_t sl = band_slot(g, A + 2 * B, args.c, it.K, it.J0 + t == g.N2 ? 0 : it.J0 + t, I);
 #pragma unroll
-            for (int c = 0; c < 3; c++) v[u][c] = __ldcs(r + sl + c * (size_t)g.npad);
+            for (int c = 0; c < 3; c++) v[u][c] = load_once(r + sl + c * (size_t)g.npad);
         }
     }
 };
@@ -683,7 +681,7 @@ struct LameRhs {
 template <int M2, int NH, int A, int B>
 __device__ __forceinline__ void lame_colour(const BandArgs &args, const LameOp<float> &op, const BandItem &it, float *s,
                                             const int (&ib)[3], int I, int hh, const LameRhs<M2, NH, A, B> &rhs,
-                                            float *__restrict__ xout) {
+                                            float *xout) {
     constexpr int rowstep = 4 * M2;
     const Geom &g = args.g;
 #pragma unroll
@@ -706,7 +704,7 @@ template <int M2, int NH>
 __global__ void __launch_bounds__(NH * M2)
     gs_band_lame_kernel(const BandArgs args, const LameOp<float> op, const __grid_constant__ BandMaps in,
                         const __grid_constant__ BandMaps out_maps, const __grid_constant__ BandMaps mu,
-                        const __grid_constant__ BandMaps lam, const float *__restrict__ r, float *__restrict__ xout) {
+                        const __grid_constant__ BandMaps lam, const float *r, float *xout) {
     extern __shared__ __align__(128) unsigned char band_smem[];
     __shared__ __align__(8) unsigned long long bar_store;
     const Geom &g = args.g;
@@ -780,9 +778,9 @@ __global__ void __launch_bounds__(NH * M2)
 // between them), in the arithmetic and order of residual_kernel
 // (const_row<T, ELASTIC, true> / plane_row_coef<T, SPARSE, true>).
 template <typename T, int M2, int KIND, bool SPARSE, int A, int B, int NR>
-__device__ __forceinline__ void band_res_colour(const T *__restrict__ s, const int (&ib)[3], const LevelOp<T> &op,
+__device__ __forceinline__ void band_res_colour(const T *s, const int (&ib)[3], const LevelOp<T> &op,
                                                 const T *cf, int t0, int nv, const Geom &g, int c, int K, int J0,
-                                                int I, const T *__restrict__ r, T *__restrict__ res) {
+                                                int I, const T *r, T *res) {
     constexpr int rowstep = woff<M2>(0, 0, 1, 0, 0);
     const size_t np = (size_t)g.npad;
     if constexpr (KIND != OP_CONST) {
@@ -896,7 +894,7 @@ __device__ __forceinline__ void band_res_colour(const T *__restrict__ s, const i
 template <typename T, int M2, int NH, int KIND, bool SPARSE, bool PAD>
 __global__ void __launch_bounds__(NH * M2, sizeof(T) == 4 && M2 >= 96 ? 2 : 1)
     residual_band_kernel(const BandArgs args, const __grid_constant__ LevelOp<T> op,
-                         const __grid_constant__ BandMaps xm, const T *__restrict__ r, T *__restrict__ res) {
+                         const __grid_constant__ BandMaps xm, const T *r, T *res) {
     extern __shared__ __align__(128) unsigned char band_smem[];
     __shared__ __align__(8) unsigned long long bar_store;
     __shared__ __align__(16) T cfs[KIND == OP_PLANE ? kCoefWords : 4];

@@ -31,8 +31,40 @@ namespace stzmg {
 // it -- and lets the one after it start when its own work is nearly done
 // (chain_next).  Let go at once, the next kernels' blocks take the places of an
 // SM unevenly (FP64 solve at 160x96x129: 48.2 ms against 44.2 and 44.9 without).
+//
+// The kernel before still writes while such a kernel runs, so nothing that a
+// kernel of the cycle writes may be promised to be constant: no __restrict__ on
+// a pointer to it (loads through one may be taken as invariant, moved ahead of
+// chain_wait and served from the read-only path), in the kernel or in a function
+// that it calls.  Coefficients, the bottom's inverse and its slots, which only
+// a set-up writes, may be.  Loads with a cache hint are written out as volatile,
+// which keeps them behind the waits and barriers that are volatile too.  (FP64
+// solve at 160x96x129: 44.1 -> 44.2 ms; the other solves as before.)
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A value that another CTA wrote, from L2.
+__device__ __forceinline__ float load_l2(const float *p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double load_l2(const double *p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+// A value that is read once.
+__device__ __forceinline__ float load_once(const float *p) {
+    float v;
+    asm volatile("ld.global.cs.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double load_once(const double *p) {
+    double v;
+    asm volatile("ld.global.cs.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 
 struct Geom {
     int m, n, o;      // nodes per dimension

@@ -127,7 +127,7 @@ struct BlockPair {
 // Colours 4c .. 4c+3 of every plane of parity c, `cl` CTAs (one cluster) per
 // plane; x is updated in place.
 __global__ void __launch_bounds__(kThreads32, 2)
-    gs_dense32_kernel(Geom g, int c, int cl, DenseOp<float> op, const float *__restrict__ r, float *x) {
+    gs_dense32_kernel(Geom g, int c, int cl, DenseOp<float> op, const float *r, float *x) {
     __shared__ DotTable dots[2];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int rank = blockIdx.x % cl, K = blockIdx.x / cl;
@@ -201,8 +201,8 @@ __global__ void __launch_bounds__(kThreads32, 2)
 // |r - A x|^2 to partial.
 template <bool NORM>
 __global__ void __launch_bounds__(kThreads32)
-    residual_dense32_kernel(Geom g, DenseOp<float> op, const float *__restrict__ r, const float *__restrict__ x,
-                            float *__restrict__ res, double *__restrict__ partial) {
+    residual_dense32_kernel(Geom g, DenseOp<float> op, const float *r, const float *x, float *res,
+                            double *partial) {
     __shared__ DotTable dots[2];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = blockIdx.x & 7;
     const bool sums = wid == kDotWarps;
@@ -342,7 +342,7 @@ __device__ __forceinline__ double row_times(const double (&m)[3], double acc, in
 }
 
 __global__ void __launch_bounds__(kThreads64)
-    gs_dense64_kernel(Geom g, int c, int cl, DenseOp<double> op, const double *__restrict__ r, double *x) {
+    gs_dense64_kernel(Geom g, int c, int cl, DenseOp<double> op, const double *r, double *x) {
     __shared__ double parts[kTeams][2][4][32];
     const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) & 3, team = threadIdx.x >> 7;
     const int row = lane / kNodes64, node = lane - kNodes64 * row;   // row 3: two idle lanes
@@ -415,8 +415,8 @@ __global__ void __launch_bounds__(kThreads64)
 
 template <typename R, bool NORM>
 __global__ void __launch_bounds__(kThreads64)
-    residual_dense64_kernel(Geom g, DenseOp<double> op, const double *__restrict__ r, const double *__restrict__ x,
-                            R *__restrict__ res, double *__restrict__ partial) {
+    residual_dense64_kernel(Geom g, DenseOp<double> op, const double *r, const double *x, R *res,
+                            double *partial) {
     __shared__ double parts[kTeams][2][4][32];
     __shared__ double red[kThreads64 / 32];
     const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) & 3, team = threadIdx.x >> 7;

@@ -32,11 +32,11 @@ __host__ __device__ constexpr bool elastic_entry(int b, int e) {
 // persistent small-level kernel), so read it through L2 (ld.global.cg), not
 // from a possibly stale L1 line.
 template <typename T, bool COH = false>
-__device__ inline void load3(const T *__restrict__ f, int npad, int s, T *v) {
+__device__ inline void load3(const T *f, int npad, int s, T *v) {
     if (COH) {
-        v[0] = __ldcg(f + s);
-        v[1] = __ldcg(f + s + npad);
-        v[2] = __ldcg(f + s + 2 * npad);
+        v[0] = load_l2(f + s);
+        v[1] = load_l2(f + s + npad);
+        v[2] = load_l2(f + s + 2 * npad);
     } else {
         v[0] = f[s];
         v[1] = f[s + npad];

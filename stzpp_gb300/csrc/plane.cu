@@ -73,7 +73,7 @@ __device__ __forceinline__ T row_part(int d, const T *cf, const LaneRow &L, cons
     const bool zin = t.oz[d] >= 0;
     auto value = [&](const T *p, bool in) {
         T v = T(0);
-        if (in) v = COH && d == 1 ? __ldcg(p) : *p;
+        if (in) v = COH && d == 1 ? load_l2(p) : *p;
         return v;
     };
     T v[9][3];
@@ -135,7 +135,7 @@ constexpr int kMaxWarps = 12;   // two CTAs share an SM: their colours' barriers
 // plane; x is updated in place.
 template <typename T>
 __global__ void __launch_bounds__(32 * kMaxWarps, 2)
-    gs_plane_rows_kernel(Geom g, int c, int cl, PlaneOp<T> op, const T *__restrict__ r, T *x) {
+    gs_plane_rows_kernel(Geom g, int c, int cl, PlaneOp<T> op, const T *r, T *x) {
     __shared__ T cf[252];
     const int lane = threadIdx.x & 31, row = min(lane / kNodes, 2), node = lane % kNodes;
     const int rank = blockIdx.x % cl, K = blockIdx.x / cl, plane = g.M2 * g.N2;
@@ -193,8 +193,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 2)
 
 // res = r - A x of plane blockIdx.y (unused slots get 0): four colours, a warp per 10 slots.
 __global__ void __launch_bounds__(256)
-    residual_plane64_kernel(Geom g, PlaneOp<double> op, const double *__restrict__ r, const double *__restrict__ x,
-                            double *__restrict__ res) {
+    residual_plane64_kernel(Geom g, PlaneOp<double> op, const double *r, const double *x, double *res) {
     __shared__ double cf[252];
     const int lane = threadIdx.x & 31, row = min(lane / kNodes, 2), node = lane % kNodes;
     const int k = blockIdx.y, c = k & 1, K = k >> 1, plane = g.M2 * g.N2, groups = (plane + kNodes - 1) / kNodes;

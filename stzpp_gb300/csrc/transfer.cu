@@ -28,7 +28,7 @@ __device__ inline bool regular_dim(int I, int mc, int mf, int prd) {
 }
 
 template <typename T>
-__global__ void restriction_kernel(Geom gf, Geom gc, const T *__restrict__ res, T *__restrict__ rc, T *__restrict__ xc) {
+__global__ void restriction_kernel(Geom gf, Geom gc, const T *res, T *rc, T *xc) {
     chain_wait();
     const int I = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y * blockDim.y + threadIdx.y, K = blockIdx.z;
     if (I >= gc.m || J >= gc.n) return;
@@ -71,7 +71,7 @@ __global__ void restriction_kernel(Geom gf, Geom gc, const T *__restrict__ res, 
 // 2c + s, s in {0,1}^3, that exist.  Every fine node belongs to exactly one
 // cell (c = f >> 1).
 template <typename T>
-__global__ void interpolation_kernel(Geom gf, Geom gc, const T *__restrict__ xc, T *__restrict__ xf) {
+__global__ void interpolation_kernel(Geom gf, Geom gc, const T *xc, T *xf) {
     chain_wait();
     const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y, ck = blockIdx.z;
     if (ci >= gc.m || cj >= gc.n) return;
@@ -229,7 +229,7 @@ constexpr int kBottomRows = 4;
 template <typename T>
 __global__ void __launch_bounds__(32 * kBottomRows)
     bottom_direct_kernel(int nrow, const double *__restrict__ ainv, const int *__restrict__ nat_slot, int npad,
-                         const T *__restrict__ r, T *__restrict__ x) {
+                         const T *r, T *x) {
     extern __shared__ double rn[];
     chain_wait();
     const int lane = threadIdx.x & 31, row = blockIdx.x * kBottomRows + (threadIdx.x >> 5);

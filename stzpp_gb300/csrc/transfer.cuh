@@ -28,7 +28,7 @@ __device__ inline int wrapi(int a, int len) {
 // Coarse r at slot p (node I,J,K) = sum of (1/8) P-weighted fine residuals,
 // including the restrict_partial mask-145 quirk (see transfer.cu).
 template <typename T, bool COH = false>
-__device__ inline void restrict_node(const Geom &gf, const Geom &gc, const T *__restrict__ res, int p, int I, int J,
+__device__ inline void restrict_node(const Geom &gf, const Geom &gc, const T *res, int p, int I, int J,
                                      int K, T *acc) {
     acc[0] = acc[1] = acc[2] = T(0);
     const bool xs = !gf.xp && !(gf.m & 1) && I == gc.m - 2;
@@ -72,7 +72,7 @@ __device__ inline int parents(int f, int mf, int mc, int prd, int *c) {
 
 // (P x_c) at fine node (i,j,k).
 template <typename T, bool COH = false>
-__device__ inline void interp_node(const Geom &gf, const Geom &gc, const T *__restrict__ xc, int i, int j, int k,
+__device__ inline void interp_node(const Geom &gf, const Geom &gc, const T *xc, int i, int j, int k,
                                    T *s) {
     int cx[2], cy[2], cz[2];
     int nx = parents(i, gf.m, gc.m, gf.xp, cx);
