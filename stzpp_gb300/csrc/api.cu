@@ -465,7 +465,8 @@ void build_bottom(stz_mg_handle h) {
     const int lb = h->nlev - 1;
     const Geom &g = h->geo[lb];
     const size_t N = npts(g);
-    if (N > 4096) fail(STZ_MG_ERR_UNSUPPORTED, "direct bottom solve limited to 4096 nodes (have %zu)", N);
+    if (N > kMaxBottomNodes)
+        fail(STZ_MG_ERR_UNSUPPORTED, "direct bottom solve limited to %d nodes (have %zu)", kMaxBottomNodes, N);
     const int nr = (int)(3 * N);
     // buffers are sized by the bottom level, which does not change between set-ups
     if (!h->ainv_t || h->nbot_rows != nr) {
@@ -528,7 +529,7 @@ void choose_tail(stz_mg_handle h) {
     int cap = 0;
     for (int l = lo; l <= L - 2; l++)
         if (h->op64[l].kind == OP_PLANE) cap = std::max(cap, h->geo[l].o);
-    const int budget = 200 * 1024;
+    const int budget = kTailSmem;
     if ((size_t)cap * 252 * tsz > (size_t)budget) cap = (int)(budget / (252 * tsz));
     const int smem = (int)(cap * 252 * tsz);
     const int cl = mixed ? tail_cluster_size<float>(smem) : tail_cluster_size<double>(smem);

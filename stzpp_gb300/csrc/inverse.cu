@@ -555,22 +555,29 @@ void eliminate(double *a, int n, double *rows, int *pivots, int *bad, cudaStream
 
 }  // namespace
 
+// Shared memory of a system of order bs: two rows and the pivots; the system
+// too, unless it works in the inverse's place, which is written last.  (With
+// three columns or more an order is at most kMaxBottomNodes.)
+static int fourier_smem(int bs) {
+    return bs * (int)(2 * sizeof(double2) + 2 * sizeof(int)) +
+           (bs <= kFourierOrder ? 2 * bs * bs * (int)sizeof(double) : 0);
+}
+
 // False where the blocks would not fit the scratch (n x n doubles): one or two
 // columns, for which the plain inverse is as good.
 bool launch_fourier_inverse(const PlaneOp<double> &op, const Geom &g, const int *S, double *inv, double *scratch,
                             int *bad, cudaStream_t st) {
     const int bs = 3 * g.o, cols = g.m * g.n, n = bs * cols;
     if (!g.xp || !g.yp || cols < 3) return false;
-    // systems beyond shared memory work in the inverse's place, which is written last
-    const bool fits = bs <= kFourierOrder;
-    const int smem = bs * (int)(2 * sizeof(double2) + 2 * sizeof(int)) + (fits ? 2 * bs * bs * (int)sizeof(double) : 0);
-    const int phases = cols * (int)sizeof(double2);   // 64 KB at the 4096 nodes a direct bottom may have
-    cudaFuncSetAttribute(fourier_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaFuncSetAttribute(fourier_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, phases);
+    const int smem = fourier_smem(bs), phases = cols * (int)sizeof(double2);
+    static SmemLimit inverse_limit, blocks_limit;
+    inverse_limit.allow(std::max(fourier_smem(kFourierOrder), fourier_smem(kMaxBottomNodes)), fourier_inverse_kernel);
+    blocks_limit.allow(kMaxBottomNodes * (int)sizeof(double2), fourier_blocks_kernel);
     double2 *G = reinterpret_cast<double2 *>(scratch);
     double *B = scratch + 2 * (size_t)cols * bs * bs;
     box_check_kernel<<<(g.m * g.n * g.o + 127) / 128, 128, 0, st>>>(g, S, bad);
-    fourier_inverse_kernel<<<cols, kFourierThreads, smem, st>>>(g, op, G, fits ? nullptr : inv, bad);
+    fourier_inverse_kernel<<<cols, kFourierThreads, smem, st>>>(g, op, G,
+                                                             bs <= kFourierOrder ? nullptr : inv, bad);
     fourier_blocks_kernel<<<dim3((bs * bs + 127) / 128, cols), 128, phases, st>>>(g.m, g.n, bs, G, B);
     fourier_expand_kernel<<<dim3((n + 255) / 256, n), 256, 0, st>>>(g, B, inv);
     return true;

@@ -1,6 +1,8 @@
 // Host-side declarations of the kernel launchers of the GB300 multigrid.
 #pragma once
 
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -8,6 +10,26 @@
 namespace stzmg {
 
 constexpr int kMaxLevels = 16;
+constexpr int kMaxBottomNodes = 4096;   // of a direct bottom solve
+
+// The limit of a kernel's dynamic shared memory belongs to the function and the
+// device, not to a launch or a handle: set to a launch's own size it would take
+// from under another thread what its larger launch needs.  So it is set once
+// per device, to the most that any launch takes, and counts as set only then.
+class SmemLimit {
+    std::atomic<unsigned long long> devices{0};
+
+public:
+    template <typename... K>
+    void allow(int bytes, K *...kernels) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const unsigned long long bit = 1ull << (dev & 63);
+        if (devices.load(std::memory_order_acquire) & bit) return;
+        if ((... && (cudaFuncSetAttribute(kernels, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)))
+            devices.fetch_or(bit, std::memory_order_release);
+    }
+};
 
 // A launch that may overlap the end of the one before it in the stream: of
 // kernels that call chain_wait (common.cuh), in clusters of `cluster` CTAs.
@@ -194,7 +216,7 @@ void launch_lame_grad(const LameOp<double> &op, const Geom &g, const double *w, 
 
 // tail.cu: persistent cluster kernels for the small levels lo..hi (hi+1 is
 // the bottom level).  Levels must be OP_PLANE or OP_DENSE.
-constexpr int kTailThreads = 1024;
+constexpr int kTailThreads = 1024, kTailSmem = 200 * 1024;
 template <typename T>
 struct TailLev {
     Geom g;

@@ -153,10 +153,10 @@ static int tail_smem_bytes(const TailDesc<T> &d) {
 template <typename T>
 static cudaError_t launch_cluster(void (*kern)(TailDesc<T>), const TailDesc<T> &d, int cluster, cudaStream_t st) {
     const int smem = tail_smem_bytes(d);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
+    static SmemLimit limit;
+    limit.allow(kTailSmem, tail_down_kernel<T>, tail_up_kernel<T>);
     if (cluster > 8) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
@@ -200,7 +200,7 @@ int tail_cluster_size(int smem_bytes) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         auto kern = tail_down_kernel<T>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) continue;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem) != cudaSuccess) continue;
         if (c > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) continue;
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1) return c;

@@ -293,9 +293,9 @@ void launch_scale(double *v, double s, size_t n, cudaStream_t st) {
 template <typename T>
 void launch_bottom_direct(int nrow, const double *ainv_t, const int *nat_slot, int npad, const T *r, T *x,
                           cudaStream_t st) {
-    const int smem = nrow * (int)sizeof(double);   // 96 KB at the 4096 nodes a direct bottom may have
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(bottom_direct_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const int smem = nrow * (int)sizeof(double);
+    static SmemLimit limit;
+    limit.allow(3 * kMaxBottomNodes * (int)sizeof(double), bottom_direct_kernel<T>);
     launch_chained(bottom_direct_kernel<T>, (nrow + kBottomRows - 1) / kBottomRows, 32 * kBottomRows, smem, st, 1, nrow,
                    ainv_t, nat_slot, npad, r, x);
 }
