@@ -1029,15 +1029,6 @@ bool make_band_maps(const Geom &g, int pad, const T *field, BandMaps &mp, int co
     return true;
 }
 
-bool first_band_use(unsigned long long &devices) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (devices & bit) return false;
-    devices |= bit;
-    return true;
-}
-
 // Threads per column of the residual kernel: two (each thread two of the
 // band's four sub-rows, which share each coefficient load; four threads with
 // one row each measured slower: level 1 59.5 against 43.9 us).
@@ -1050,8 +1041,8 @@ bool launch_band_kn(const LevelOp<T> &op, const Geom &g, const T *r, const T *xi
     if (!make_band_maps<T>(g, M2, xin, min_) || !make_band_maps<T>(g, M2, xout, mout)) return false;
     auto kern = gs_band_kernel<T, M2, NH, KIND, SPARSE, PAD>;
     const int smem = kBandWords<M2> * (int)sizeof(T);
-    static unsigned long long attr_devices = 0;
-    if (first_band_use(attr_devices)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static SmemLimit limit;   // per instantiation
+    limit.allow(smem, kern);
     BandArgs a;
     a.g = g;
     a.nbands = g.n / band_rows(g.M2);
@@ -1128,8 +1119,8 @@ bool launch_band_lame_m(const LameOp<float> &op, const Geom &g, const float *r, 
         return false;
     auto kern = gs_band_lame_kernel<M2, NH>;
     const int smem = kLameWords<M2> * (int)sizeof(float);
-    static unsigned long long attr_devices = 0;
-    if (first_band_use(attr_devices)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static SmemLimit limit;   // per instantiation
+    limit.allow(smem, kern);
     BandArgs a;
     a.g = g;
     a.nbands = g.n / band_rows(g.M2);
@@ -1209,8 +1200,8 @@ bool launch_res_band_k(const LevelOp<T> &op, const Geom &g, const T *r, const T 
     constexpr int NH = kResNH<T, M2>;
     auto kern = residual_band_kernel<T, M2, NH, KIND, SPARSE, PAD>;
     const int smem = kBandWords<M2> * (int)sizeof(T);
-    static unsigned long long attr_devices = 0;
-    if (first_band_use(attr_devices)) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static SmemLimit limit;   // per instantiation
+    limit.allow(smem, kern);
     BandArgs a;
     a.g = g;
     a.nbands = g.n / band_rows(g.M2);

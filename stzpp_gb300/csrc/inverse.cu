@@ -473,7 +473,8 @@ __global__ void bottom_matrix_kernel(Geom g, const double *__restrict__ coef, co
 template <int W>
 int panel_ctas(int n) {
     cudaFuncSetAttribute(gj_panel_kernel<W>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    cudaFuncSetAttribute(gj_panel_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPanelSmem);
+    static SmemLimit limit;
+    limit.allow(kPanelSmem, gj_panel_kernel<W>);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(16);
     cfg.blockDim = dim3(kPanelThreads);

@@ -151,10 +151,15 @@ static int tail_smem_bytes(const TailDesc<T> &d) {
 }
 
 template <typename T>
-static cudaError_t launch_cluster(void (*kern)(TailDesc<T>), const TailDesc<T> &d, int cluster, cudaStream_t st) {
-    const int smem = tail_smem_bytes(d);
+static void allow_tail_smem() {
     static SmemLimit limit;
     limit.allow(kTailSmem, tail_down_kernel<T>, tail_up_kernel<T>);
+}
+
+template <typename T>
+static cudaError_t launch_cluster(void (*kern)(TailDesc<T>), const TailDesc<T> &d, int cluster, cudaStream_t st) {
+    const int smem = tail_smem_bytes(d);
+    allow_tail_smem<T>();
     if (cluster > 8) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e != cudaSuccess) return e;
@@ -200,7 +205,7 @@ int tail_cluster_size(int smem_bytes) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         auto kern = tail_down_kernel<T>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem) != cudaSuccess) continue;
+        allow_tail_smem<T>();
         if (c > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) continue;
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1) return c;
