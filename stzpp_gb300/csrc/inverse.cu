@@ -293,10 +293,20 @@ __global__ void gj_gather_kernel(const double *__restrict__ a, int n, const int 
 //     D(t) = sum_d A(d) e^{i t.d},  t = 2 pi (kx / m, ky / n),
 // and the inverse couples the columns through B(d) = 1/(m n) sum_t D(t)^-1
 // e^{-i t.d}.  A CTA per t builds D(t) from the planes' rows and inverts it in
-// shared memory by the same elimination as above.  On the host, one system
-// after the other, 64 systems of order 27 took 11.6 ms; here 134 us.
+// shared memory by the same elimination as above; a column's magnitudes are
+// compared by their squares unless those leave the exponent range.  On the host,
+// one system after the other, 64 systems of order 27 took 11.6 ms; here 134 us.
 constexpr int kFourierThreads = 256;
 constexpr int kFourierOrder = 104;   // two arrays of order^2 doubles in shared memory
+
+// Squares of magnitudes in here are far from the ends of the exponent range.
+constexpr long long kSmallSquare = (1023ll - 900) << 52, kLargeSquare = (1023ll + 900) << 52;
+
+// 2^-n for a value of about 2^n, within the range where both are normal numbers.
+__device__ __forceinline__ double unit_of(double v) {
+    const int n = (int)(magnitude(v) >> 52) - 1023;
+    return __longlong_as_double((long long)(1023 - max(-1000, min(1000, n))) << 52);
+}
 
 // work: null, or 2 bs^2 doubles per CTA for systems beyond shared memory.
 __global__ void __launch_bounds__(kFourierThreads)
@@ -309,7 +319,7 @@ __global__ void __launch_bounds__(kFourierThreads)
                       : reinterpret_cast<double *>(smem + (size_t)bs * (2 * sizeof(double2) + 2 * sizeof(int)));
     double *im = re + bs * bs;
     __shared__ double2 wx[3], wy[3];
-    __shared__ int piv;
+    __shared__ int piv, far;   // the pivot's row, and whether its square is out of range
     if (tid < 6) {   // e^{i t d}
         const int d = tid % 3 - 1;
         double sn, cs;
@@ -334,30 +344,40 @@ __global__ void __launch_bounds__(kFourierThreads)
     __syncthreads();
     for (int c = 0; c < bs; c++) {
         if (tid < 32) {
-            long long best = -1;
-            int at = c;
-            for (int r = c + tid; r < bs; r += 32) {
-                const double u = re[r * bs + c], v = im[r * bs + c];
-                const long long q = magnitude(u * u + v * v);
-                if (q > best) best = q, at = r;
-            }
+            long long best;
+            int at;
+            auto search = [&](auto size) {
+                best = -1, at = c;
+                for (int r = c + tid; r < bs; r += 32) {
+                    const long long q = magnitude(size(re[r * bs + c], im[r * bs + c]));
+                    if (q > best) best = q, at = r;
+                }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const long long v = __shfl_down_sync(0xffffffffu, best, o);
-                const int j = __shfl_down_sync(0xffffffffu, at, o);
-                if (better(v, j, best, at)) best = v, at = j;
-            }
+                for (int o = 16; o > 0; o >>= 1) {
+                    const long long v = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int j = __shfl_xor_sync(0xffffffffu, at, o);
+                    if (better(v, j, best, at)) best = v, at = j;
+                }
+            };
+            search([](double u, double v) { return u * u + v * v; });
+            const bool extreme = best < kSmallSquare || best > kLargeSquare;
+            if (extreme) search([](double u, double v) { return hypot(u, v); });
             if (tid == 0) {
                 piv = pivots[c] = at;
+                far = extreme;
                 if (no_pivot(best)) atomicExch(bad, 1);
             }
         }
         __syncthreads();
         // swap rows c and piv; the pivot row over the pivot, and column c
         const int p = piv;
-        const double pr = re[p * bs + c], pi = im[p * bs + c];
+        const double unit = far ? unit_of(fmax(fabs(re[p * bs + c]), fabs(im[p * bs + c]))) : 1.0;
+        double pr = re[p * bs + c], pi = im[p * bs + c];
+        if (far) pr *= unit, pi *= unit;
         for (int e = tid; e < bs; e += kFourierThreads) {
-            const double s2 = 1.0 / (pr * pr + pi * pi), ir = pr * s2, ii = -pi * s2;
+            const double s2 = 1.0 / (pr * pr + pi * pi);
+            double ir = pr * s2, ii = -pi * s2;
+            if (far) ir *= unit, ii *= unit;
             const double ur = re[p * bs + e], ui = im[p * bs + e];
             prow[e] = e == c ? make_double2(ir, ii) : make_double2(ur * ir - ui * ii, ur * ii + ui * ir);
             const int r = e == p ? c : e;   // the row whose values are at e after the swap
