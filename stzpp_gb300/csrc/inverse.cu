@@ -64,13 +64,19 @@ __device__ __forceinline__ bool better(long long m, int i, long long than, int a
     return m > than || (m == than && (unsigned)i < (unsigned)at);
 }
 
-// 1/v to within an ulp or two, by two Newton steps from FP32's reciprocal: five
-// FP64 instructions on the elimination's critical path, where the division is
-// twice that.  Values out of FP32's range take the division.
+// 1/v, correctly rounded, by Newton steps from FP32's reciprocal: six
+// FP64 instructions on the elimination's critical path, fewer than the division.
+// Two steps leave less than an ulp of error, from where a third one rounds
+// correctly unless v's significand is all ones (P. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34,
+// 1990); without it reciprocals next to the middle between two doubles are off.
+// That significand and values out of FP32's range take the division.
 __device__ __forceinline__ double reciprocal(double v) {
-    const unsigned e = (unsigned)(__double_as_longlong(v) >> 52) & 0x7ff;
-    if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / v;
+    const long long b = __double_as_longlong(v), ones = (1ll << 52) - 1;
+    const unsigned e = (unsigned)(b >> 52) & 0x7ff;
+    if (e < 1023 - 100 || e > 1023 + 100 || (b & ones) == ones) return 1.0 / v;
     double y = (double)(1.0f / (float)v);
+    y = fma_rn(fma_rn(-v, y, 1.0), y, y);
     y = fma_rn(fma_rn(-v, y, 1.0), y, y);
     return fma_rn(fma_rn(-v, y, 1.0), y, y);
 }
