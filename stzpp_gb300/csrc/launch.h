@@ -2,6 +2,7 @@
 #pragma once
 
 #include <atomic>
+#include <utility>
 
 #include <cuda_runtime.h>
 
@@ -33,6 +34,8 @@ public:
 
 // A launch that may overlap the end of the one before it in the stream: of
 // kernels that call chain_wait (common.cuh), in clusters of `cluster` CTAs.
+// Arguments convert to the kernel's parameters as in a call: by no cast that
+// would make one pointer out of another.
 template <typename... P, typename... A>
 inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster,
                            A &&...args) {
@@ -49,7 +52,7 @@ inline void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
     at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 // One level's operator as the kernels see it.
