@@ -33,8 +33,8 @@
 //  * a quotient by a parameter takes five instructions (quotient_by);
 //  * cells above the yield stress are collected per block and sub-stepped by
 //    full warps, a lane taking the next cell when its own is done.
-// 256^3 cells, 23 % above the yield stress: update 23.1 -> 14.2 ms, plastic
-// 6.0 -> 2.0 ms; 48x40x24 cells: 107 -> 51 and 42 -> 24 us.
+// 256^3 cells, 23 % above the yield stress: update 23.1 -> 13.3 ms, plastic
+// 6.0 -> 2.0 ms; 48x40x24 cells: 107 -> 50 and 42 -> 25 us.
 #include <cuda_runtime.h>
 
 #include "stz_mg.h"

@@ -93,9 +93,10 @@ template <typename T>
 bool gs_tile_applies(const LevelOp<T> &op, const Geom &g);
 template <typename T>
 void launch_gs_sweep_tile(const LevelOp<T> &op, const Geom &g, const T *r, const T *xin, T *xout, cudaStream_t st);
-// band.cu: one sweep reading xin and writing xout on the top level of a
-// shared elasticity stencil periodic in x, y (full-width bands of 8 rows,
-// planes staged by TMA); false if the tensor maps cannot be made
+// band.cu: one sweep reading xin and writing xout on a level periodic in x, y
+// of up to 256 nodes a row -- a shared stencil, a plane-invariant operator or
+// FP32 Lame coefficients (full-width bands of 8 rows, planes staged by TMA);
+// false if the tensor maps cannot be made
 template <typename T>
 bool gs_band_applies(const LevelOp<T> &op, const Geom &g);
 template <typename T>

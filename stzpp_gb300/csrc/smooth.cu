@@ -335,8 +335,10 @@ void launch_gs_sweeps(const LevelOp<T> &op, const Geom &g, const T *r, T *x, T *
     int s = 0;
     // pairs of sweeps x -> tmp -> x by the tiled kernel (tile.cu), which needs
     // a second buffer; a last odd sweep in place (same result either way)
-    // plane-invariant levels of 64x64 and more: 4+ tiles per plane beat one
-    // block per plane (64x64x65, two FP32 sweeps: 58 vs 107 us); 32x32 does not
+    // plane-invariant levels of 64x64 nodes a plane and more have four tiles and
+    // more a plane, which beat a cluster a plane (plane.cu): two FP32 sweeps of
+    // 64x64x65, 32x128x33 or 128x32x33 41 against 88 us.  (The bands take these
+    // levels unless STZ_MG_BAND=0 or a row has more than 256 nodes.)
     const bool plane_tiles = op.kind == OP_PLANE && g.m * g.n >= 64 * 64;
     // shared stencils and plane-invariant levels: full-width bands whose planes
     // arrive by TMA (band.cu); a last odd sweep comes back by a copy, which is
